@@ -86,6 +86,11 @@ namespace sint
                                                 cudaStream_t, const ResidualHooks *);
 
   // --- dispatch over (dim, mobility) ---------------------------------------
+  static bool runs_fused(const Ctx *c, size_t real_size)
+  {
+    return !c->cut && !c->adv && runs_fused2d(c->grid.dim, c->G, c->params.tensorial != 0, real_size);
+  }
+
   template <typename R>
   cudaError_t dispatch_jvp(const Ctx *c, const R *lin, const R *src, R *dst, cudaStream_t s)
   {
@@ -102,8 +107,9 @@ namespace sint
             : launch_jvp<2, false, R>(c->G, c->grid, c->phys, lin, src, dst, part, cut, adv, s);
     if (e != cudaSuccess)
       return e;
-    e = c->grid.dim == 3 ? launch_combine<3, R>(c->C, c->grid, part, dst, active_tile_union(c), s, nullptr)
-                         : launch_combine<2, R>(c->C, c->grid, part, dst, active_tile_union(c), s, nullptr);
+    if (!runs_fused(c, sizeof(R)))
+      e = c->grid.dim == 3 ? launch_combine<3, R>(c->C, c->grid, part, dst, active_tile_union(c), s, nullptr)
+                           : launch_combine<2, R>(c->C, c->grid, part, dst, active_tile_union(c), s, nullptr);
     if (e != cudaSuccess)
       return e;
     return launch_periodic_condense<R>(c->grid, c->C, dst, src, 0, s);
@@ -139,8 +145,10 @@ namespace sint
             : launch_residual<2, false>(c->G, wtd, c->grid, ph, src, hist, dst, c->partial, cut, adv, s);
     if (e != cudaSuccess)
       return e;
-    e = c->grid.dim == 3 ? launch_combine<3, double>(c->C, c->grid, c->partial, dst, active_tile_union(c), s, &ph.hooks)
-                         : launch_combine<2, double>(c->C, c->grid, c->partial, dst, active_tile_union(c), s, &ph.hooks);
+    if (!runs_fused(c, sizeof(double)))
+      e = c->grid.dim == 3 ?
+            launch_combine<3, double>(c->C, c->grid, c->partial, dst, active_tile_union(c), s, &ph.hooks) :
+            launch_combine<2, double>(c->C, c->grid, c->partial, dst, active_tile_union(c), s, &ph.hooks);
     if (e != cudaSuccess)
       return e;
     if ((e = launch_periodic_condense<double>(c->grid, c->C, dst, nullptr, 1, s)) != cudaSuccess || !epi_after)

@@ -181,8 +181,76 @@ namespace sint
     P[(res * Slots<DIM>::NQ + q) * Tile<DIM>::CELLS + cell] = v;
   }
 
-  // Phase 2 of the Jacobian product at point q of cell `cell`
-  // (SinteringOperatorGenericQuad::operator(), generic.h:101-190).
+  // Point terms of the Jacobian product (SinteringOperatorGenericQuad::
+  // operator(), generic.h:101-190) from the fields at one point: the state
+  // (c, eta and their gradients, grad mu), and the direction (d*).  Every
+  // result goes to emit(res, value) with pstore's numbering: res 0 = c row
+  // value, 1..DIM = c row flux, DIM + 1 = mu row value, DIM + 2 + i = eta_i
+  // row value.
+  template <int DIM, int G, bool TENS, typename R, typename Emit>
+  __device__ __forceinline__ void jvp_terms(const PhysR<R> &p, const R &c, const R (&gc)[DIM], const R (&gmu)[DIM],
+                                            const R (&eta)[gdim(G)], const R (*geta)[DIM], const R &dc,
+                                            const R (&gdc)[DIM], const R &dmu, const R (&gdmu)[DIM],
+                                            const R (&deta)[gdim(G)], unsigned m, Emit emit)
+  {
+    // free energy second derivatives at the linearisation point (free_energy.h:143-161)
+    R s2 = R(0);
+#pragma unroll
+    for (int i = 0; i < G; ++i)
+      s2 += eta[i] * eta[i];
+    const R omc = R(1) - c;
+    const R fcc = R(2) * p.A * (c * c) + R(4) * p.A * c * (R(2) * c - R(2)) + R(2) * p.A * (omc * omc) + R(2) * p.B;
+    const R B12 = p.B * R(12);
+    // f_{c eta_i} = 12 B eta_i (eta_i - 1) (free_energy.h:150-152), shared by the mu
+    // and eta rows; f_{eta_i eta_i} = B (12 - 12 c + 2 eta_i (12 c - 24) + 24 eta_i^2
+    // + 12 sum eta^2) (:154-158) in Horner form: f0 + eta_i (f1 + f2 eta_i)
+    R fce[gdim(G)];
+#pragma unroll
+    for (int i = 0; i < G; ++i)
+      {
+        const R be = B12 * eta[i];
+        fce[i]     = be * eta[i] - be;
+      }
+    const R fee0 = B12 * ((R(1) - c) + s2), fee1 = p.B * (R(24) * c - R(48)), fee2 = p.B * R(24);
+
+    // 1) c row (generic.h:120-134)
+    {
+      R gres[DIM];
+      apply_M_derivative<DIM, G, TENS>(p, c, gc, gmu, eta, geta, dc, gdc, gdmu, deta, gres, m);
+      emit(0, dc * p.w0);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        emit(1 + d, gres[d]);
+    }
+    // 2) mu row value (generic.h:138-144)
+    {
+      R v = p.walg * dmu - fcc * dc;
+#pragma unroll
+      for (int i = 0; i < G; ++i)
+        v -= fce[i] * deta[i];
+      emit(DIM + 1, v);
+    }
+    // 3) eta row values (generic.h:150-163, free_energy.h:233-252)
+    {
+      R S = R(0);
+#pragma unroll
+      for (int i = 0; i < G; ++i)
+        S += eta[i] * deta[i];
+      const R cL24B = p.L * R(24) * p.B;
+#pragma unroll
+      for (int i = 0; i < G; ++i)
+        {
+          const R e   = eta[i];
+          const R fee = fee0 + e * (fee1 + fee2 * e);
+          R       v   = deta[i] * p.w0 + p.L * (fce[i] * dc + fee * deta[i]);
+          if constexpr (G > 1)
+            v += (cL24B * e) * (S - e * deta[i]);
+          emit(DIM + 2 + i, v);
+        }
+    }
+  }
+
+  // Phase 2 of the Jacobian product at point q of cell `cell`.
   template <int DIM, int G, bool TENS, typename R>
   __device__ __forceinline__ void jvp_point(const PhysR<R> &p, const R *F, R *P, int q, int cell, unsigned m = ~0u)
   {
@@ -211,66 +279,53 @@ namespace sint
 #pragma unroll
     for (int i = 0; i < G; ++i)
       deta[i] = fval<DIM>(F, FM::base(FM::src_eta(i)), q, cell);
+    jvp_terms<DIM, G, TENS, R>(p, c, gc, gmu, eta, geta, dc, gdc, dmu, gdmu, deta, m,
+                               [&](int res, R v) { pstore<DIM>(P, res, q, cell, v); });
+  }
 
-    // free energy second derivatives at the linearisation point (free_energy.h:143-161)
-    R s2 = R(0);
-#pragma unroll
-    for (int i = 0; i < G; ++i)
-      s2 += eta[i] * eta[i];
-    const R omc = R(1) - c;
-    const R fcc = R(2) * p.A * (c * c) + R(4) * p.A * c * (R(2) * c - R(2)) + R(2) * p.A * (omc * omc) + R(2) * p.B;
-    const R B12 = p.B * R(12);
-    // f_{c eta_i} = 12 B eta_i (eta_i - 1) (free_energy.h:150-152), shared by the mu
-    // and eta rows; f_{eta_i eta_i} = B (12 - 12 c + 2 eta_i (12 c - 24) + 24 eta_i^2
-    // + 12 sum eta^2) (:154-158) in Horner form: f0 + eta_i (f1 + f2 eta_i)
-    R fce[gdim(G)];
+  // Point terms of the residual (SinteringOperatorGenericResidualQuad::
+  // operator(), generic.h:254-308) from the fields at one point;
+  // time(i, v) adds the time-derivative term of c (i = -1) or eta_i to v,
+  // emit(res, value) as in jvp_terms.
+  template <int DIM, int G, bool TENS, typename R, typename Time, typename Emit>
+  __device__ __forceinline__ void residual_terms(const PhysR<R> &p, const R &c, const R (&gc)[DIM], const R &mu,
+                                                 const R (&gmu)[DIM], const R (&eta)[gdim(G)], const R (*geta)[DIM],
+                                                 unsigned m, Time time, Emit emit)
+  {
+    R s2 = R(0), s3 = R(0);
 #pragma unroll
     for (int i = 0; i < G; ++i)
       {
-        const R be = B12 * eta[i];
-        fce[i]     = be * eta[i] - be;
+        s2 += eta[i] * eta[i];
+        s3 += eta[i] * eta[i] * eta[i];
       }
-    const R fee0 = B12 * ((R(1) - c) + s2), fee1 = p.B * (R(24) * c - R(48)), fee2 = p.B * R(24);
-
-    // 1) c row (generic.h:120-134)
+    const R omc = R(1) - c;
+    // 1) c row (generic.h:275-285)
     {
-      R gres[DIM];
-      apply_M_derivative<DIM, G, TENS>(p, c, gc, gmu, eta, geta, dc, gdc, gdmu, deta, gres, m);
-      pstore<DIM>(P, 0, q, cell, dc * p.w0);
+      const R v = time(-1, R(0));
+      R       gres[DIM];
+      apply_M<DIM, G, TENS>(p, c, eta, gc, geta, gmu, gres, m);
+      emit(0, v);
 #pragma unroll
       for (int d = 0; d < DIM; ++d)
-        pstore<DIM>(P, 1 + d, q, cell, gres[d]);
+        emit(1 + d, gres[d]);
     }
-    // 2) mu row value (generic.h:138-144)
+    // 2) mu row value (generic.h:288, free_energy.h:124-134)
     {
-      R v = p.walg * dmu - fcc * dc;
-#pragma unroll
-      for (int i = 0; i < G; ++i)
-        v -= fce[i] * deta[i];
-      pstore<DIM>(P, DIM + 1, q, cell, v);
+      const R df_dc = p.A * (c * c) * (R(2) * c - R(2)) + R(2) * p.A * c * (omc * omc) +
+                      p.B * (R(2) * c - R(6) * s2 + R(4) * s3);
+      emit(DIM + 1, p.walg * mu - df_dc);
     }
-    // 3) eta row values (generic.h:150-163, free_energy.h:233-252)
-    {
-      R S = R(0);
+    // 3) eta row values (generic.h:293-302, free_energy.h:136-141)
 #pragma unroll
-      for (int i = 0; i < G; ++i)
-        S += eta[i] * deta[i];
-      const R cL24B = p.L * R(24) * p.B;
-#pragma unroll
-      for (int i = 0; i < G; ++i)
-        {
-          const R e   = eta[i];
-          const R fee = fee0 + e * (fee1 + fee2 * e);
-          R       v   = deta[i] * p.w0 + p.L * (fce[i] * dc + fee * deta[i]);
-          if constexpr (G > 1)
-            v += (cL24B * e) * (S - e * deta[i]);
-          pstore<DIM>(P, DIM + 2 + i, q, cell, v);
-        }
-    }
+    for (int i = 0; i < G; ++i)
+      {
+        const R e = eta[i];
+        emit(DIM + 2 + i, time(i, p.L * (e * (p.B * R(12)) * (e * (c - R(2)) + omc + s2))));
+      }
   }
 
-  // Phase 2 of the residual at point q of cell `cell`
-  // (SinteringOperatorGenericResidualQuad::operator(), generic.h:254-308).
+  // Phase 2 of the residual at point q of cell `cell`.
   template <int DIM, int G, bool TENS, int WTD, typename R>
   __device__ __forceinline__ void residual_point(const PhysR<R> &p, const R *F, R *P, int q, int cell,
                                                  unsigned m = ~0u)
@@ -291,46 +346,16 @@ namespace sint
         if constexpr (TENS)
           fgrad<DIM>(F, FM::base(FM::lin_eta(i)), q, cell, geta[i]);
       }
-    R s2 = R(0), s3 = R(0);
-#pragma unroll
-    for (int i = 0; i < G; ++i)
-      {
-        s2 += eta[i] * eta[i];
-        s3 += eta[i] * eta[i] * eta[i];
-      }
-    const R omc = R(1) - c;
-    // 1) c row (generic.h:275-285)
-    {
-      R v = R(0);
-      if constexpr (WTD >= 1)
-        v = c * p.w0;
-      if constexpr (WTD == 2)
-        v += fval<DIM>(F, FM::base(FM::h_c), q, cell);
-      R gres[DIM];
-      apply_M<DIM, G, TENS>(p, c, eta, gc, geta, gmu, gres, m);
-      pstore<DIM>(P, 0, q, cell, v);
-#pragma unroll
-      for (int d = 0; d < DIM; ++d)
-        pstore<DIM>(P, 1 + d, q, cell, gres[d]);
-    }
-    // 2) mu row value (generic.h:288, free_energy.h:124-134)
-    {
-      const R df_dc = p.A * (c * c) * (R(2) * c - R(2)) + R(2) * p.A * c * (omc * omc) +
-                      p.B * (R(2) * c - R(6) * s2 + R(4) * s3);
-      pstore<DIM>(P, DIM + 1, q, cell, p.walg * mu - df_dc);
-    }
-    // 3) eta row values (generic.h:293-302, free_energy.h:136-141)
-#pragma unroll
-    for (int i = 0; i < G; ++i)
-      {
-        const R e = eta[i];
-        R       v = p.L * (e * (p.B * R(12)) * (e * (c - R(2)) + omc + s2));
+    residual_terms<DIM, G, TENS, R>(
+      p, c, gc, mu, gmu, eta, geta, m,
+      [&](int i, R v) {
         if constexpr (WTD >= 1)
-          v += e * p.w0;
+          v += (i < 0 ? c : eta[i < 0 ? 0 : i]) * p.w0;
         if constexpr (WTD == 2)
-          v += fval<DIM>(F, FM::base(FM::h_eta(i)), q, cell);
-        pstore<DIM>(P, DIM + 2 + i, q, cell, v);
-      }
+          v += fval<DIM>(F, FM::base(i < 0 ? FM::h_c : FM::h_eta(i)), q, cell);
+        return v;
+      },
+      [&](int res, R v) { pstore<DIM>(P, res, q, cell, v); });
   }
 
   // Global coordinates of local cell `cell` of tile tc; false outside the mesh.

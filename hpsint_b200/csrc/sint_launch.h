@@ -42,6 +42,18 @@ namespace sint
     return cudaSuccess;
   }
 
+  // Whether the full operator (no cut-off, no advection) runs as one kernel
+  // that finishes every node itself (sint_fused2d.cuh): no tile-face
+  // partials, no combine step.  In 2D always, but for the FP64 tensorial
+  // operator of more than 10 grains: its point physics and row sums spill at
+  // 255 registers, and the tiled kernels are faster on small meshes (256 x
+  // 128 cells, G = 12: residual 51.6 us tiled, 57.8 us fused; J v 58.1 /
+  // 59.8; G = 10: 41.3 / 41.3 and 45.3 / 43.3).
+  constexpr bool runs_fused2d(int dim, int G, bool tensorial, size_t real_size)
+  {
+    return dim == 2 && !(real_size == 8 && tensorial && G > 10);
+  }
+
   // Dynamic shared memory of the diagonal kernel (bytes); adv: with the
   // grains' velocities per point.
   size_t smem_diag(int dim, int G, bool adv = false);

@@ -4,6 +4,7 @@
 #pragma once
 #include <type_traits>
 
+#include "sint_fused2d.cuh"
 #include "sint_kernels.cuh"
 #include "sint_launch.h"
 
@@ -105,6 +106,27 @@ namespace sint
     return cudaGetLastError();
   }
 
+  // The one-kernel 2D cell loop (MODE: -1 = J v, 0..2 = residual).
+  template <int G, bool TENS, typename R, int MODE>
+  cudaError_t launch_fused2d_g(const Grid &g, const Phys &p, Fused2DArgs<R> args, cudaStream_t s)
+  {
+    using L           = Fused2D<G, MODE>;
+    const size_t smem = L::template smem<R>();
+    auto         k    = fused2d_kernel<G, TENS, R, MODE>;
+    static DeviceCache cache;
+    int                ready = 0;
+    if (const cudaError_t e = per_device(cache, ready, [&](int, int &v) {
+          v = 1;
+          return prepare_smem(k, smem, fused2d_blocks<G, TENS, R>());
+        }))
+      return e;
+    args.blocks_x          = (g.nn[0] + L::TX - 2) / (L::TX - 1);
+    const long long blocks = (long long)args.blocks_x * ((g.nn[1] + L::TY - 2) / (L::TY - 1));
+    k<<<dim3((unsigned)blocks), L::THREADS, smem, s>>>(g, p, args);
+    count_launches(1);
+    return cudaGetLastError();
+  }
+
   template <int DIM, int G, bool TENS, bool CUT, bool ADV>
   cudaError_t launch_diag_g(const Grid &g, const Phys &p, const double *lin, double *dst, double *partial,
                             const uint16_t *mask, const AdvData &adv, cudaStream_t s)
@@ -171,6 +193,20 @@ namespace sint
 #undef SINT_CALL
   }
 
+  // The full operator's J v: one kernel in 2D (sint_fused2d.cuh), packed FP32
+  // tile pairs, or the tiled kernel.
+  template <int DIM, int G, bool TENS, typename R, bool ADV>
+  cudaError_t launch_jvp_full(const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
+                              const AdvData &adv, cudaStream_t s)
+  {
+    if constexpr (!ADV && runs_fused2d(DIM, G, TENS, sizeof(R)))
+      return launch_fused2d_g<G, TENS, R, -1>(g, p, Fused2DArgs<R>{lin, src, {}, dst, 0}, s);
+    else if constexpr (!ADV && std::is_same_v<R, float>)
+      return launch_jvp_pair_g<DIM, G, TENS>(g, p, lin, src, dst, partial, s);
+    else
+      return launch_jvp_g<DIM, G, TENS, R, false, ADV>(g, p, lin, src, dst, partial, CutTiles(), adv, s);
+  }
+
   // cut == nullptr: the full operator; otherwise the grain cut-off, one
   // launch per grain-count class 0..G (classes without tiles return at once).
   // ADV: the kernels with the advection terms.
@@ -186,20 +222,9 @@ namespace sint
             return e;
         return cudaSuccess;
       }
-    if constexpr (std::is_same_v<R, float> && !ADV)
-      {
-        // the full FP32 operator runs on tile pairs (packed FP32)
-#define SINT_CALL(GG) launch_jvp_pair_g<DIM, GG, TENS>(g, p, lin, src, dst, partial, s)
-        SINT_G_SWITCH(SINT_CALL)
+#define SINT_CALL(GG) launch_jvp_full<DIM, GG, TENS, R, ADV>(g, p, lin, src, dst, partial, adv, s)
+    SINT_G_SWITCH(SINT_CALL)
 #undef SINT_CALL
-      }
-    else
-      {
-        const CutTiles none;
-#define SINT_CALL(GG) launch_jvp_g<DIM, GG, TENS, R, false, ADV>(g, p, lin, src, dst, partial, none, adv, s)
-        SINT_G_SWITCH(SINT_CALL)
-#undef SINT_CALL
-      }
   }
 
   // The advection kernels are instantiated in their own translation units
@@ -213,22 +238,40 @@ namespace sint
     return launch_jvp_impl<DIM, TENS, R, false>(G, g, p, lin, src, dst, partial, cut, AdvData(), s);
   }
 
+  // The full operator's residual: one kernel in 2D, else the tiled kernel.
+  template <int DIM, int G, bool TENS, int WTD, bool ADV>
+  cudaError_t launch_residual_full(const Grid &g, const Phys &p, const double *src, const double *const *hist,
+                                   double *dst, double *partial, const AdvData &adv, cudaStream_t s)
+  {
+    if constexpr (!ADV && runs_fused2d(DIM, G, TENS, sizeof(double)))
+      {
+        Fused2DArgs<double> args{src, nullptr, {}, dst, 0};
+        for (int i = 0; WTD == 2 && i < p.order; ++i)
+          args.h[i] = hist[i];
+        return launch_fused2d_g<G, TENS, double, WTD>(g, p, args, s);
+      }
+    else
+      return launch_residual_g<DIM, G, TENS, WTD, false, ADV>(g, p, src, hist, dst, partial, CutTiles(), adv, s);
+  }
+
   // G = the grain count (full operator, 1..12) or the class (grain cut-off, 0..12)
   template <int DIM, bool TENS, bool CUT, int WTD, bool ADV>
   cudaError_t launch_residual_w(int G, const Grid &g, const Phys &p, const double *src, const double *const *hist,
                                 double *dst, double *partial, const CutTiles &ct, const AdvData &adv,
                                 cudaStream_t s)
   {
-#define SINT_CALL(GG) launch_residual_g<DIM, GG, TENS, WTD, CUT, ADV>(g, p, src, hist, dst, partial, ct, adv, s)
     if constexpr (CUT)
       {
+#define SINT_CALL(GG) launch_residual_g<DIM, GG, TENS, WTD, true, ADV>(g, p, src, hist, dst, partial, ct, adv, s)
         SINT_CLASS_SWITCH(G, SINT_CALL)
+#undef SINT_CALL
       }
     else
       {
+#define SINT_CALL(GG) launch_residual_full<DIM, GG, TENS, WTD, ADV>(g, p, src, hist, dst, partial, adv, s)
         SINT_G_SWITCH(SINT_CALL)
-      }
 #undef SINT_CALL
+      }
   }
 
   template <int DIM, bool TENS, bool CUT, bool ADV>

@@ -243,14 +243,13 @@ namespace sint
     const R omc = R(1) - c;
     if constexpr (!TENS)
       {
+        // sum_{i>j} eta_i eta_j = sum_i eta_i (eta_0 + .. + eta_{i-1})
         R eta_sum = R(0), eta_ij = R(0);
 #pragma unroll
         for (int i = 0; i < G; ++i)
           {
+            eta_ij += eta[i] * eta_sum;
             eta_sum += eta[i];
-#pragma unroll
-            for (int j = 0; j < i; ++j)
-              eta_ij += eta[i] * eta[j];
           }
         const R M = p.Mvol * phi + p.Mvap * (R(1) - phi) + p.Msurf * R(4) * c * c * omc * omc + (R(2) * p.Mgb) * eta_ij;
         const R dphidc = R(30) * c * c * omc * omc;
