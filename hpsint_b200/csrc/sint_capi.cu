@@ -463,8 +463,7 @@ int sint_destroy(sint_ctx *c)
   cudaFree(c->adv_slots);
   cudaFree(c->ch_A64);
   cudaFree(c->ch_A32);
-  cudaFree(c->ch_dinv64);
-  cudaFree(c->ch_dinv32);
+  cudaFree(c->ch_scratch);
   cudaFree(c->pc_raw);
   cudaFree(c->pc_inv64);
   cudaFree(c->pc_inv32);
@@ -673,21 +672,25 @@ int sint_precond_setup(sint_ctx *c, sint_stream_t stream)
       set_error("sint_precond_setup: no linearisation point set");
       return SINT_ERR_NOT_READY;
     }
-  cudaError_t e = dispatch_diag(c, c->pc_raw, stream);
-  if (e != cudaSuccess)
-    return cuda_fail(e, "sint_precond_setup: diagonal");
-  const long long nb = (c->N + 255) / 256;
-  precond_invert_kernel<<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_raw, c->pc_inv64,
-                                                                c->pc_inv32);
-  count_launches(1);
-  if ((e = cudaGetLastError()) != cudaSuccess)
-    return cuda_fail(e, "sint_precond_setup: invert");
   c->has_ch = false;
   if (c->pc_kind == 1)
     {
+      // the Cahn-Hilliard matrix, and from the same passes the grains' diagonal
       if (int rc = ch_sgs_setup(c, stream))
         return rc;
       c->has_ch = true;
+    }
+  else
+    {
+      cudaError_t e = dispatch_diag(c, c->pc_raw, stream);
+      if (e != cudaSuccess)
+        return cuda_fail(e, "sint_precond_setup: diagonal");
+      const long long nb = (c->N + 255) / 256;
+      precond_invert_kernel<<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_raw, c->pc_inv64,
+                                                                    c->pc_inv32);
+      count_launches(1);
+      if ((e = cudaGetLastError()) != cudaSuccess)
+        return cuda_fail(e, "sint_precond_setup: invert");
     }
   c->has_pc = true;
   return SINT_OK;
@@ -720,9 +723,7 @@ int sint_ch_matrix_f64(sint_ctx *c, double *A, sint_stream_t stream)
     }
   if (int e = check_vec(A, "A"))
     return e;
-  const size_t nk = c->grid.dim == 3 ? 27 : 9;
-  const cudaError_t e =
-    cudaMemcpyAsync(A, c->ch_A64, sizeof(double) * nk * 4 * c->ld, cudaMemcpyDeviceToDevice, stream);
+  const cudaError_t e = ch_matrix_export(c, A, stream);
   return e == cudaSuccess ? SINT_OK : cuda_fail(e, "sint_ch_matrix_f64");
 }
 
@@ -739,12 +740,16 @@ int sint_precond_apply_f64(sint_ctx *c, double *z, const double *r, sint_stream_
     return e;
   if (int e = check_vec(r, "r"))
     return e;
-  const long long nb = (c->N + 255) / 256;
-  precond_apply_kernel<double><<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_inv64, r, z);
-  count_launches(1);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess && c->has_ch) // Cahn-Hilliard block by the Gauss-Seidel sweeps
+  cudaError_t e = cudaSuccess;
+  if (c->has_ch) // Cahn-Hilliard block by the Gauss-Seidel sweeps
     e = ch_sgs_apply<double>(c, r, z, stream);
+  else
+    {
+      const long long nb = (c->N + 255) / 256;
+      precond_apply_kernel<double><<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_inv64, r, z);
+      count_launches(1);
+      e = cudaGetLastError();
+    }
   return e == cudaSuccess ? SINT_OK : cuda_fail(e, "sint_precond_apply_f64");
 }
 
@@ -761,12 +766,16 @@ int sint_precond_apply_f32(sint_ctx *c, float *z, const float *r, sint_stream_t 
     return e;
   if (int e = check_vec(r, "r"))
     return e;
-  const long long nb = (c->N + 255) / 256;
-  precond_apply_kernel<float><<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_inv32, r, z);
-  count_launches(1);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess && c->has_ch) // Cahn-Hilliard block by the Gauss-Seidel sweeps
+  cudaError_t e = cudaSuccess;
+  if (c->has_ch) // Cahn-Hilliard block by the Gauss-Seidel sweeps
     e = ch_sgs_apply<float>(c, r, z, stream);
+  else
+    {
+      const long long nb = (c->N + 255) / 256;
+      precond_apply_kernel<float><<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_inv32, r, z);
+      count_launches(1);
+      e = cudaGetLastError();
+    }
   return e == cudaSuccess ? SINT_OK : cuda_fail(e, "sint_precond_apply_f32");
 }
 

@@ -487,9 +487,11 @@ namespace sint
     // box offsets of the nodes l xor x of this lane's node l (stiffness stencil)
     int koff[1 << DIM];
 
-    __device__ __forceinline__ explicit QP(const Grid &g)
+    __device__ __forceinline__ explicit QP(const Grid &g) : QP(g, threadIdx.x & ((1 << DIM) - 1)) {}
+
+    __device__ __forceinline__ QP(const Grid &g, int point)
     {
-      q                 = threadIdx.x & ((1 << DIM) - 1);
+      q                 = point;
       const double s3   = 0.5 / 1.7320508075688772935274463415058723669428; // 1 / (2 sqrt 3)
       const double gg0  = 0.5 - s3, gg1 = 0.5 + s3;
       g1                = R(gg1);

@@ -94,10 +94,9 @@ namespace sint
     // 1 = symmetric Gauss-Seidel on the assembled block (sint_chsgs.cu)
     int     pc_kind   = 0;
     bool    has_ch    = false;   // the assembled block belongs to the current set-up
-    double *ch_A64    = nullptr; // 3^dim x 4 blocks of ld: 2x2 blocks per node row and neighbour
-    float  *ch_A32    = nullptr;
-    double *ch_dinv64 = nullptr; // 4 blocks of ld: inverted centre blocks
-    float  *ch_dinv32 = nullptr;
+    double *ch_A64     = nullptr; // 2x2 blocks of the node rows, layout and slots in sint_chsgs.cu
+    float  *ch_A32     = nullptr;
+    double *ch_scratch = nullptr; // element-matrix rows of a slab of cell layers (assembly)
 
     double *pc_raw   = nullptr; // (G+4) blocks: CH 2x2 entries, AC diagonal
     double *pc_inv64 = nullptr; // (G+4) blocks: CH 2x2 inverse, AC inverse diagonal
@@ -168,11 +167,14 @@ namespace sint
   // u, then the velocity table (sint_advection.cu).
   int advection_update(Ctx *c, const double *u, cudaStream_t s);
   // The assembled Cahn-Hilliard block and its Gauss-Seidel sweeps
-  // (sint_chsgs.cu): set-up at the linearisation point, and z_(c,mu) =
-  // SGS(r_(c,mu)) on the first two blocks of z (the others untouched).
+  // (sint_chsgs.cu): set-up at the linearisation point (with the Allen-Cahn
+  // diagonal, and the centre blocks in pc_raw), z = P^-1 r with the sweeps on
+  // the first two blocks and the inverse diagonal on the others, and the
+  // matrix in the interface's order.
   int ch_sgs_setup(Ctx *c, cudaStream_t s);
   template <typename R>
   cudaError_t ch_sgs_apply(const Ctx *c, const R *r, R *z, cudaStream_t s);
+  cudaError_t ch_matrix_export(const Ctx *c, double *A, cudaStream_t s);
   // J v through the cell kernel + combine, with c->partial as scratch.
   template <typename R>
   cudaError_t dispatch_jvp(const Ctx *c, const R *lin, const R *src, R *dst, cudaStream_t s);

@@ -400,9 +400,10 @@ namespace sint
 #pragma unroll
               for (int b = 0; b < DIM; ++b)
                 acc[a][b] = R(0);
-#pragma unroll 1
+// a loop over many grains keeps its operands in local memory, unrolled in registers
+#pragma unroll(G <= 6 ? G : 1)
             for (int i = 0; i < G; ++i)
-#pragma unroll 1
+#pragma unroll(G <= 6 ? G : 1)
               for (int j = 0; j < i; ++j)
                 {
                   R dd[DIM];
