@@ -7,6 +7,7 @@
 #include "sint_fused2d.cuh"
 #include "sint_kernels.cuh"
 #include "sint_launch.h"
+#include "sint_light.cuh"
 
 namespace sint
 {
@@ -106,6 +107,26 @@ namespace sint
     return cudaGetLastError();
   }
 
+  // The 3D class of the grain cut-off without a relevant grain (MODE: -1 = J v,
+  // 0..2 = residual); the class size lives on the device, so the grid is the
+  // persistent one.
+  template <bool TENS, typename R, int MODE>
+  cudaError_t launch_light(const Grid &g, const Phys &p, const LightArgs<R> &args, const CutTiles &ct, cudaStream_t s)
+  {
+    using L           = LightTile<MODE>;
+    const size_t smem = L::template smem<R>();
+    auto         k    = light_kernel<TENS, R, MODE>;
+    static DeviceCache cache;
+    int                grid_cap = 0;
+    if (const cudaError_t e = persistent_grid(cache, k, smem, light_blocks<R, MODE>(), L::WARPS * 32, grid_cap))
+      return e;
+    const long long need   = (g.n_tiles + L::WARPS - 1) / L::WARPS;
+    const long long blocks = need < grid_cap ? need : grid_cap;
+    k<<<dim3((unsigned)blocks), L::WARPS * 32, smem, s>>>(g, p, args, ct);
+    count_launches(1);
+    return cudaGetLastError();
+  }
+
   // The one-kernel 2D cell loop (MODE: -1 = J v, 0..2 = residual).
   template <int G, bool TENS, typename R, int MODE>
   cudaError_t launch_fused2d_g(const Grid &g, const Phys &p, Fused2DArgs<R> args, cudaStream_t s)
@@ -183,10 +204,12 @@ namespace sint
   cudaError_t launch_jvp_class(int K, const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
                                const CutTiles &ct, const AdvData &adv, cudaStream_t s)
   {
-    // FP32: the class without grains (c and mu only, the bulk of a packing's
-    // vapour) runs on tile pairs
-    if constexpr (std::is_same_v<R, float> && !ADV)
+    // the class without grains (c and mu only, the bulk of a packing's vapour)
+    if constexpr (DIM == 3 && !ADV)
       if (K == 0)
+        return launch_light<TENS, R, -1>(g, p, LightArgs<R>{lin, src, {}, dst, partial}, ct, s);
+    if constexpr (DIM == 2 && std::is_same_v<R, float> && !ADV)
+      if (K == 0) // on tile pairs
         return launch_jvp_pair_g<DIM, 0, TENS, true>(g, p, lin, src, dst, partial, s, ct);
 #define SINT_CALL(GG) launch_jvp_g<DIM, GG, TENS, R, true, ADV>(g, p, lin, src, dst, partial, ct, adv, s)
     SINT_CLASS_SWITCH(K, SINT_CALL)
@@ -262,6 +285,14 @@ namespace sint
   {
     if constexpr (CUT)
       {
+        if constexpr (DIM == 3 && !ADV)
+          if (G == 0)
+            {
+              LightArgs<double> args{src, nullptr, {}, dst, partial};
+              for (int i = 0; WTD == 2 && i < p.order; ++i)
+                args.h[i] = hist[i];
+              return launch_light<TENS, double, WTD>(g, p, args, ct, s);
+            }
 #define SINT_CALL(GG) launch_residual_g<DIM, GG, TENS, WTD, true, ADV>(g, p, src, hist, dst, partial, ct, adv, s)
         SINT_CLASS_SWITCH(G, SINT_CALL)
 #undef SINT_CALL
