@@ -76,11 +76,11 @@ namespace sint
       u[l] = s[b0 + (l & 1) + T::SY * ((l >> 1) & 1) + (DIM == 3 ? T::SZ * ((l >> 2) & 1) : 0)];
   }
 
-  // Phase 1, value + gradient: writes F[(base + slot) * CELLS + cell] for the
-  // NQ values followed by DIM blocks of NG1 gradient slots.
+  // Phase 1, value + gradient: writes F[(slot) * CELLS + cell] for the NQ
+  // values from slot base on and DIM blocks of NG1 gradient slots from gbase on.
   template <int DIM, typename R>
   __device__ __forceinline__ void cell_eval_vg(const R (&u)[1 << DIM], const CellConsts<DIM, R> &k, R *F, int base,
-                                               int cell)
+                                               int gbase, int cell)
   {
     constexpr int CELLS = Tile<DIM>::CELLS;
     const R       xq[2] = {k.x0, k.x1};
@@ -125,7 +125,7 @@ namespace sint
 #pragma unroll
               for (int qz = 0; qz < 2; ++qz)
                 F[(base + qx + 2 * qy + 4 * qz) * CELLS + cell] = vxy[0][qy][qx] + xq[qz] * d;
-              F[(base + 8 + 8 + qx + 2 * qy) * CELLS + cell] = d * k.ih[2]; // d/dz at (qy, qx)
+              F[(gbase + 8 + qx + 2 * qy) * CELLS + cell] = d * k.ih[2]; // d/dz at (qy, qx)
             }
 #pragma unroll
         for (int qy = 0; qy < 2; ++qy)
@@ -133,7 +133,7 @@ namespace sint
             const R dd = dxy[1][qy] - dxy[0][qy];
 #pragma unroll
             for (int qz = 0; qz < 2; ++qz)
-              F[(base + 8 + qy + 2 * qz) * CELLS + cell] = (dxy[0][qy] + xq[qz] * dd) * k.ih[0]; // d/dx at (qz, qy)
+              F[(gbase + qy + 2 * qz) * CELLS + cell] = (dxy[0][qy] + xq[qz] * dd) * k.ih[0]; // d/dx at (qz, qy)
           }
 #pragma unroll
         for (int qx = 0; qx < 2; ++qx)
@@ -141,7 +141,7 @@ namespace sint
             const R dd = dyl[1][qx] - dyl[0][qx];
 #pragma unroll
             for (int qz = 0; qz < 2; ++qz)
-              F[(base + 8 + 4 + qx + 2 * qz) * CELLS + cell] = (dyl[0][qx] + xq[qz] * dd) * k.ih[1]; // d/dy at (qz, qx)
+              F[(gbase + 4 + qx + 2 * qz) * CELLS + cell] = (dyl[0][qx] + xq[qz] * dd) * k.ih[1]; // d/dy at (qz, qx)
           }
       }
     else
@@ -163,12 +163,12 @@ namespace sint
 #pragma unroll
             for (int qy = 0; qy < 2; ++qy)
               F[(base + qx + 2 * qy) * CELLS + cell] = vx[0][qx] + xq[qy] * d;
-            F[(base + 4 + 2 + qx) * CELLS + cell] = d * k.ih[1]; // d/dy at qx
+            F[(gbase + 2 + qx) * CELLS + cell] = d * k.ih[1]; // d/dy at qx
           }
         const R dd = dxl[1] - dxl[0];
 #pragma unroll
         for (int qy = 0; qy < 2; ++qy)
-          F[(base + 4 + qy) * CELLS + cell] = (dxl[0] + xq[qy] * dd) * k.ih[0]; // d/dx at qy
+          F[(gbase + qy) * CELLS + cell] = (dxl[0] + xq[qy] * dd) * k.ih[0]; // d/dx at qy
       }
   }
 

@@ -42,18 +42,28 @@ namespace sint
   // Residual (u = the state, h = the weighted history):
   //   tensorial: [c, mu, eta_i] (value + gradient), [h c, h eta_i] (value)
   //   scalar:    [mu] (value + gradient), [c, eta_i] (value), [h c, h eta_i] (value)
-  template <int DIM, int G, bool TENS, bool JVP, bool HIST>
+  template <int DIM, int G, bool TENS, bool JVP, bool HIST, bool IN_PLACE = false>
   struct FieldMap
   {
     using SL = Slots<DIM>;
     static constexpr int NVG    = JVP ? (TENS ? 4 + G : 2) : (TENS ? 2 + G : 1);
     static constexpr int NV     = JVP ? (TENS ? G : 2 + 2 * G) : ((TENS ? 0 : 1 + G) + (HIST ? 1 + G : 0));
     static constexpr int NITEMS = NVG + NV;
-    static constexpr int NSLOT  = NVG * SL::VG + NV * SL::V;
+    // slots: the values of all items first, then the gradients of the first
+    // NVG; with IN_PLACE at least as many value slots as there are point results
+    static constexpr int NRES  = DIM + 2 + G;
+    static constexpr int NVAL  = IN_PLACE && NRES > NITEMS ? NRES : NITEMS;
+    static constexpr int NSLOT = NVAL * SL::V + NVG * (SL::VG - SL::V);
 
-    __host__ __device__ static constexpr int base(int item)
+    __host__ __device__ static constexpr int base(int item) { return item * SL::V; }
+    __host__ __device__ static constexpr int gbase(int item) { return NVAL * SL::V + item * (SL::VG - SL::V); }
+    // Value slot (in units of NQ) of point result res.  IN_PLACE: results
+    // replace values that only the same (point, cell) thread reads: the eta_i
+    // row eta_i's own, the others (written last) the values before the first
+    // and behind the last eta_i; together the first NRES slots.
+    __host__ __device__ static constexpr int result(int res)
     {
-      return item < NVG ? item * SL::VG : NVG * SL::VG + (item - NVG) * SL::V;
+      return !IN_PLACE ? res : (res >= DIM + 2 ? lin_eta(res - DIM - 2) : (res < lin_eta(0) ? res : G + res));
     }
     // item index of each quantity (residual: "lin" is the state itself)
     static constexpr int lin_c  = TENS ? 0 : (JVP ? 2 : 1);
@@ -118,13 +128,13 @@ namespace sint
   // the items of a grain absent on this thread's cell (bit clear in m) are
   // zero; a warp that has no lane needing an item writes the zeros without
   // evaluating.
-  template <int DIM, int G, bool TENS, bool JVP, bool HIST, typename R, bool CUT = false>
+  template <int DIM, int G, bool TENS, bool JVP, bool HIST, typename R, bool CUT = false, bool IN_PLACE = false>
   __device__ __forceinline__ void phase_evaluate(const R *box0, const R *box1, R *F, const CellConsts<DIM, R> &k,
                                                  unsigned m = ~0u)
   {
     using T            = Tile<DIM>;
     using SL           = Slots<DIM>;
-    using FM           = FieldMap<DIM, G, TENS, JVP, HIST>;
+    using FM           = FieldMap<DIM, G, TENS, JVP, HIST, IN_PLACE>;
     constexpr int NGRP = T::THREADS / T::CELLS;
     const int     cell = threadIdx.x % T::CELLS;
     const int     b0   = cell_box_base<DIM>(cell);
@@ -137,9 +147,11 @@ namespace sint
             absent       = gr >= 0 && ((m >> gr) & 1u) == 0u;
             if (!__any_sync(0xffffffffu, !absent))
               {
-                const int ns = it < FM::NVG ? SL::VG : SL::V;
-                for (int sl = 0; sl < ns; ++sl)
+                for (int sl = 0; sl < SL::V; ++sl)
                   F[(FM::base(it) + sl) * T::CELLS + cell] = R(0);
+                if (it < FM::NVG)
+                  for (int sl = 0; sl < SL::VG - SL::V; ++sl)
+                    F[(FM::gbase(it) + sl) * T::CELLS + cell] = R(0);
                 continue;
               }
           }
@@ -153,7 +165,7 @@ namespace sint
             for (int l = 0; l < (1 << DIM); ++l)
               u[l] = R(0);
         if (it < FM::NVG)
-          cell_eval_vg<DIM>(u, k, F, FM::base(it), cell);
+          cell_eval_vg<DIM>(u, k, F, FM::base(it), FM::gbase(it), cell);
         else
           cell_eval_v<DIM>(u, k, F, FM::base(it), cell);
       }
@@ -166,14 +178,14 @@ namespace sint
     return F[(base + q) * Tile<DIM>::CELLS + cell];
   }
   template <int DIM, typename R>
-  __device__ __forceinline__ void fgrad(const R *F, int base, int q, int cell, R (&g)[DIM])
+  __device__ __forceinline__ void fgrad(const R *F, int gbase, int q, int cell, R (&g)[DIM])
   {
 #pragma unroll
     for (int d = 0; d < DIM; ++d)
-      g[d] = F[(base + Slots<DIM>::NQ + d * Slots<DIM>::NG1 + grad_slot<DIM>(d, q)) * Tile<DIM>::CELLS + cell];
+      g[d] = F[(gbase + d * Slots<DIM>::NG1 + grad_slot<DIM>(d, q)) * Tile<DIM>::CELLS + cell];
   }
 
-  // point results: P[(res * NQ + q) * CELLS + cell]; res 0 = c row value,
+  // point results: P[(FieldMap::result(res) * NQ + q) * CELLS + cell]; res 0 = c row value,
   // 1..DIM = c row flux, DIM + 1 = mu row value, DIM + 2 + i = eta_i row value
   template <int DIM, typename R>
   __device__ __forceinline__ void pstore(R *P, int res, int q, int cell, nd<R> v)
@@ -251,15 +263,14 @@ namespace sint
   }
 
   // Phase 2 of the Jacobian product at point q of cell `cell`.
-  template <int DIM, int G, bool TENS, typename R>
+  template <int DIM, int G, bool TENS, typename FM, typename R>
   __device__ __forceinline__ void jvp_point(const PhysR<R> &p, const R *F, R *P, int q, int cell, unsigned m = ~0u)
   {
-    using FM = FieldMap<DIM, G, TENS, true, false>;
     R c, gc[DIM], gmu[DIM];
     c = fval<DIM>(F, FM::base(FM::lin_c), q, cell);
     if constexpr (TENS)
-      fgrad<DIM>(F, FM::base(FM::lin_c), q, cell, gc);
-    fgrad<DIM>(F, FM::base(FM::lin_mu), q, cell, gmu);
+      fgrad<DIM>(F, FM::gbase(FM::lin_c), q, cell, gc);
+    fgrad<DIM>(F, FM::gbase(FM::lin_mu), q, cell, gmu);
     R eta[gdim(G)];
     R geta[TENS ? gdim(G) : 1][DIM];
 #pragma unroll
@@ -267,20 +278,20 @@ namespace sint
       {
         eta[i] = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
         if constexpr (TENS)
-          fgrad<DIM>(F, FM::base(FM::lin_eta(i)), q, cell, geta[i]);
+          fgrad<DIM>(F, FM::gbase(FM::lin_eta(i)), q, cell, geta[i]);
       }
     R dc, gdc[DIM], dmu, gdmu[DIM];
     dc = fval<DIM>(F, FM::base(FM::src_c), q, cell);
     if constexpr (TENS)
-      fgrad<DIM>(F, FM::base(FM::src_c), q, cell, gdc);
+      fgrad<DIM>(F, FM::gbase(FM::src_c), q, cell, gdc);
     dmu = fval<DIM>(F, FM::base(FM::src_mu), q, cell);
-    fgrad<DIM>(F, FM::base(FM::src_mu), q, cell, gdmu);
+    fgrad<DIM>(F, FM::gbase(FM::src_mu), q, cell, gdmu);
     R deta[gdim(G)];
 #pragma unroll
     for (int i = 0; i < G; ++i)
       deta[i] = fval<DIM>(F, FM::base(FM::src_eta(i)), q, cell);
     jvp_terms<DIM, G, TENS, R>(p, c, gc, gmu, eta, geta, dc, gdc, dmu, gdmu, deta, m,
-                               [&](int res, R v) { pstore<DIM>(P, res, q, cell, v); });
+                               [&](int res, R v) { pstore<DIM>(P, FM::result(res), q, cell, v); });
   }
 
   // Point terms of the residual (SinteringOperatorGenericResidualQuad::
@@ -326,17 +337,16 @@ namespace sint
   }
 
   // Phase 2 of the residual at point q of cell `cell`.
-  template <int DIM, int G, bool TENS, int WTD, typename R>
+  template <int DIM, int G, bool TENS, int WTD, typename FM, typename R>
   __device__ __forceinline__ void residual_point(const PhysR<R> &p, const R *F, R *P, int q, int cell,
                                                  unsigned m = ~0u)
   {
-    using FM = FieldMap<DIM, G, TENS, false, WTD == 2>;
     R c, gc[DIM], mu, gmu[DIM];
     c = fval<DIM>(F, FM::base(FM::lin_c), q, cell);
     if constexpr (TENS)
-      fgrad<DIM>(F, FM::base(FM::lin_c), q, cell, gc);
+      fgrad<DIM>(F, FM::gbase(FM::lin_c), q, cell, gc);
     mu = fval<DIM>(F, FM::base(FM::lin_mu), q, cell);
-    fgrad<DIM>(F, FM::base(FM::lin_mu), q, cell, gmu);
+    fgrad<DIM>(F, FM::gbase(FM::lin_mu), q, cell, gmu);
     R eta[gdim(G)];
     R geta[TENS ? gdim(G) : 1][DIM];
 #pragma unroll
@@ -344,7 +354,7 @@ namespace sint
       {
         eta[i] = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
         if constexpr (TENS)
-          fgrad<DIM>(F, FM::base(FM::lin_eta(i)), q, cell, geta[i]);
+          fgrad<DIM>(F, FM::gbase(FM::lin_eta(i)), q, cell, geta[i]);
       }
     residual_terms<DIM, G, TENS, R>(
       p, c, gc, mu, gmu, eta, geta, m,
@@ -355,7 +365,160 @@ namespace sint
           v += fval<DIM>(F, FM::base(i < 0 ? FM::h_c : FM::h_eta(i)), q, cell);
         return v;
       },
-      [&](int res, R v) { pstore<DIM>(P, res, q, cell, v); });
+      [&](int res, R v) { pstore<DIM>(P, FM::result(res), q, cell, v); });
+  }
+
+  // ---- the residual of many grains in 3D: pair sums streamed from shared memory
+  // With more than 5 grains the state of a point does not fit 128 registers,
+  // and one block of 256 threads per SM (8 warps) left the residual waiting on
+  // latency (9 grains: issue in 24 % of the cycles).  Here a point thread
+  // keeps a block of pair_block grains in registers and streams the others
+  // past it, and the results replace values in the point-field buffer
+  // (FieldMap IN_PLACE), so that two blocks fit an SM's registers and shared
+  // memory: 96^3 cells, BDF2, 9 grains 1794 -> 1203 us (tensorial), 1450 ->
+  // 864 us (scalar).  The FP64 Jacobian product was not faster this way (9
+  // grains 1178 -> 1231 us: the streamed operands are 40 % more) and keeps
+  // its registers.
+  template <int G>
+  __host__ __device__ constexpr int pair_block()
+  {
+    return G % 3 == 0 && G % 4 != 0 ? 3 : 4;
+  }
+
+  template <int DIM, typename R>
+  struct PairGrain
+  {
+    R e, g[DIM];
+
+    template <typename FM>
+    __device__ __forceinline__ void load(const R *F, int i, int q, int cell)
+    {
+      e = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
+      fgrad<DIM>(F, FM::gbase(FM::lin_eta(i)), q, cell, g);
+    }
+  };
+
+  // s1 = sum_{i>j} eta_i eta_j and acc = -sum_{i>j} eta_i eta_j f_ij d_ij (d_ij .
+  // grad mu), the projected part of the pair mobility (mobility.h:785-804)
+  template <int DIM, int G, typename FM, typename R>
+  __device__ __forceinline__ void pair_sums(const R *F, int q, int cell, const R (&gmu)[DIM], unsigned m, R &s1,
+                                            R (&acc)[DIM])
+  {
+    constexpr int BI = pair_block<G>();
+    s1               = R(0);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d)
+      acc[d] = R(0);
+    auto pair = [&](const PairGrain<DIM, R> &x, const PairGrain<DIM, R> &y) {
+      R dd[DIM];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        dd[d] = x.g[d] - y.g[d];
+      const R p1 = x.e * y.e;
+      s1 += p1;
+      const R t = p1 * unit_vector_filter_2<DIM>(dd) * dotv<DIM>(dd, gmu);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        acc[d] -= t * dd[d];
+    };
+#pragma unroll 1
+    for (int i0 = 0; i0 < G; i0 += BI)
+      {
+        PairGrain<DIM, R> x[BI];
+#pragma unroll
+        for (int b = 0; b < BI; ++b)
+          if (G % BI == 0 || i0 + b < G)
+            x[b].template load<FM>(F, i0 + b, q, cell);
+#pragma unroll
+        for (int b = 1; b < BI; ++b)
+          if (G % BI == 0 || i0 + b < G)
+#pragma unroll
+            for (int c = 0; c < b; ++c)
+              if (pair_needed(m, i0 + b, i0 + c))
+                pair(x[b], x[c]);
+#pragma unroll 1
+        for (int j = 0; j < i0; ++j)
+          {
+            PairGrain<DIM, R> y;
+            y.template load<FM>(F, j, q, cell);
+#pragma unroll
+            for (int b = 0; b < BI; ++b)
+              if (G % BI == 0 || i0 + b < G)
+                if (pair_needed(m, i0 + b, j))
+                  pair(x[b], y);
+          }
+      }
+  }
+
+  // residual_point with the pair sums streamed and the results in place.
+  template <int DIM, int G, bool TENS, int WTD, typename FM, typename R>
+  __device__ __forceinline__ void residual_point_streamed(const PhysR<R> &p, R *F, int q, int cell, unsigned m)
+  {
+    const R c = fval<DIM>(F, FM::base(FM::lin_c), q, cell), mu = fval<DIM>(F, FM::base(FM::lin_mu), q, cell);
+    R       flux[DIM];
+    {
+      R gc[DIM], gmu[DIM], none[1] = {R(0)};
+      const R(*gnone)[DIM] = nullptr;
+      fgrad<DIM>(F, FM::gbase(FM::lin_mu), q, cell, gmu);
+      if constexpr (TENS)
+        {
+          R s1, acc[DIM];
+          pair_sums<DIM, G, FM>(F, q, cell, gmu, m, s1, acc);
+          fgrad<DIM>(F, FM::gbase(FM::lin_c), q, cell, gc);
+          apply_M<DIM, 1, TENS>(p, c, none, gc, gnone, gmu, flux); // the c part
+          const R m2 = R(2) * p.Mgb;
+#pragma unroll
+          for (int d = 0; d < DIM; ++d)
+            flux[d] += m2 * (s1 * gmu[d] + acc[d]);
+        }
+      else
+        {
+          R etaij = R(0), sum = R(0); // sum_i eta_i (eta_0 + .. + eta_{i-1})
+#pragma unroll 3
+          for (int i = 0; i < G; ++i)
+            {
+              const R e = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
+              etaij += e * sum;
+              sum += e;
+            }
+          apply_M<DIM, 1, TENS>(p, c, none, gc, gnone, gmu, flux);
+#pragma unroll
+          for (int d = 0; d < DIM; ++d)
+            flux[d] += ((R(2) * p.Mgb) * etaij) * gmu[d];
+        }
+    }
+    R v0 = R(0);
+    if constexpr (WTD >= 1)
+      v0 = c * p.w0;
+    if constexpr (WTD == 2)
+      v0 += fval<DIM>(F, FM::base(FM::h_c), q, cell);
+    R s2 = R(0), s3 = R(0);
+#pragma unroll 3
+    for (int i = 0; i < G; ++i)
+      {
+        const R e = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
+        s2 += e * e;
+        s3 += e * e * e;
+      }
+    const R omc = R(1) - c;
+#pragma unroll 3
+    for (int i = 0; i < G; ++i)
+      {
+        const R e = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
+        R       v = p.L * (e * (p.B * R(12)) * (e * (c - R(2)) + omc + s2));
+        if constexpr (WTD >= 1)
+          v += e * p.w0;
+        if constexpr (WTD == 2)
+          v += fval<DIM>(F, FM::base(FM::h_eta(i)), q, cell);
+        pstore<DIM>(F, FM::result(DIM + 2 + i), q, cell, v);
+      }
+    const R df_dc = p.A * (c * c) * (R(2) * c - R(2)) + R(2) * p.A * c * (omc * omc) +
+                    p.B * (R(2) * c - R(6) * s2 + R(4) * s3);
+    pstore<DIM>(F, FM::result(0), q, cell, v0);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d)
+      pstore<DIM>(F, FM::result(1 + d), q, cell, flux[d]);
+    pstore<DIM>(F, FM::result(DIM + 1), q, cell, p.walg * mu - df_dc);
   }
 
   // Global coordinates of local cell `cell` of tile tc; false outside the mesh.
@@ -469,7 +632,8 @@ namespace sint
 
   // Phase 3, 3D: the c row's contributions to the local nodes with z bit HZ
   // (K rows l = lx + 2 ly + 4 HZ) from the point values and fluxes in P.
-  template <int HZ, typename R>
+  // FM: the kernel's FieldMap (where the point results are).
+  template <int HZ, typename FM, typename R>
   __device__ __forceinline__ void integrate_c_row_half(const R *P, const CellConsts<3, R> &k, int cell, bool in,
                                                        bool in_b, R *K)
   {
@@ -479,10 +643,10 @@ namespace sint
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
       {
-        v[q] = P[(0 * NQ + q) * T::CELLS + cell];
+        v[q] = P[(FM::result(0) * NQ + q) * T::CELLS + cell];
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-          gg[d][q] = P[((1 + d) * NQ + q) * T::CELLS + cell];
+          gg[d][q] = P[(FM::result(1 + d) * NQ + q) * T::CELLS + cell];
       }
     cell_integrate_vg_half<HZ>(v, gg, k, r);
 #pragma unroll
@@ -503,7 +667,7 @@ namespace sint
   // warps in which no cell of the row moves keep the value-only integration.
   // tc_b (packed pairs only): the tile of lane y, whose cells outside the
   // mesh are zeroed lane by lane.
-  template <int DIM, int G, typename R, bool CUT = false, bool ADV = false>
+  template <int DIM, int G, typename FM, typename R, bool CUT = false, bool ADV = false>
   __device__ __forceinline__ void phase_integrate(const PhysR<R> &p, const Grid &g, const CellConsts<DIM, R> &k,
                                                   const TileCoord &tc, const R *P, const R *stiff, R *K,
                                                   unsigned m = ~0u, const R *vel = nullptr,
@@ -530,9 +694,9 @@ namespace sint
           if (task < 2)
             {
               if (task == 0)
-                integrate_c_row_half<0>(P, k, cell, in, in_b, K);
+                integrate_c_row_half<0, FM>(P, k, cell, in, in_b, K);
               else
-                integrate_c_row_half<1>(P, k, cell, in, in_b, K);
+                integrate_c_row_half<1, FM>(P, k, cell, in, in_b, K);
               continue;
             }
         bool keep = in;
@@ -555,10 +719,10 @@ namespace sint
 #pragma unroll
             for (int q = 0; q < NQ; ++q)
               {
-                v[q] = P[(0 * NQ + q) * T::CELLS + cell];
+                v[q] = P[(FM::result(0) * NQ + q) * T::CELLS + cell];
 #pragma unroll
                 for (int d = 0; d < DIM; ++d)
-                  gg[d][q] = P[((1 + d) * NQ + q) * T::CELLS + cell];
+                  gg[d][q] = P[(FM::result(1 + d) * NQ + q) * T::CELLS + cell];
               }
             cell_integrate_vg<DIM>(v, gg, k, r);
           }
@@ -595,7 +759,8 @@ namespace sint
           }
         else
           {
-            const int res = DIM + row; // mu row: DIM + 1, eta_i row (row = 2 + i): DIM + 2 + i
+            // mu row: result DIM + 1, eta_i row (row = 2 + i): DIM + 2 + i
+            const int res = FM::result(DIM + row);
             R         v[NQ];
 #pragma unroll
             for (int q = 0; q < NQ; ++q)
@@ -652,25 +817,54 @@ namespace sint
     return r;
   }
 
-  template <int DIM, int G, bool TENS, bool JVP, bool HIST, bool ADV = false>
-  struct ThreePhaseSmem
+  // Shared memory of a block (in elements) with NBUF box buffers.  IN_PLACE:
+  // the point results take the first FM::NRES value slots and the node
+  // contributions follow them, all inside the point-field buffer.
+  template <int DIM, int G, bool TENS, bool JVP, bool HIST, bool ADV, bool IN_PLACE, int NBUF>
+  struct ThreePhaseLayout
   {
     using T                     = Tile<DIM>;
-    using FM                    = FieldMap<DIM, G, TENS, JVP, HIST>;
+    using FM                    = FieldMap<DIM, G, TENS, JVP, HIST, IN_PLACE>;
     static constexpr int C      = G + 2;
     static constexpr int NQ     = 1 << DIM;
-    static constexpr int BOXES  = 2 * C * T::BOXS;                 // both inputs of one tile
-    static constexpr int F_SIZE = FM::NSLOT * T::CELLS;            // point fields (K aliases it)
-    static constexpr int P_SIZE = (DIM + 2 + G) * NQ * T::CELLS;   // point results
+    static constexpr int BOXES  = 2 * C * T::BOXS; // both inputs of one tile
     static constexpr int K_SIZE = C * NQ * T::CP;
-    static_assert(K_SIZE <= F_SIZE, "node contributions must fit in the point-field buffer");
+    static constexpr int P_AT   = IN_PLACE ? 0 : FM::NSLOT * T::CELLS;
+    static constexpr int K_AT   = IN_PLACE ? FM::NRES * NQ * T::CELLS : 0; // else aliases the dead point fields
+    static constexpr int FIELDS = FM::NSLOT * T::CELLS;
+    static constexpr int F_SIZE = IN_PLACE && K_AT + K_SIZE > FIELDS ? K_AT + K_SIZE : FIELDS;
+    static constexpr int P_SIZE = IN_PLACE ? 0 : FM::NRES * NQ * T::CELLS;
+    static_assert(IN_PLACE || K_SIZE <= F_SIZE, "node contributions must fit in the point-field buffer");
     // staged advection coefficients (adv_stage): 6 values and one flag byte
     // per (grain, cell); the flags are counted in 4-byte elements
     static constexpr int ADV_VEL = ADV ? 6 * G * T::CELLS : 0;
     static constexpr int ADV_HAS = ADV ? (G * T::CELLS + 3) / 4 : 0;
-    // elements: the JVP double-buffers its boxes, the residual does not
-    static constexpr int TOTAL = (JVP ? 2 : 1) * BOXES + F_SIZE + P_SIZE + ADV_VEL + ADV_HAS;
+    static constexpr int BUFFERS = NBUF;
+    static constexpr int TOTAL   = NBUF * BOXES + F_SIZE + P_SIZE + ADV_VEL + ADV_HAS;
   };
+
+  // Bytes a block may take for two blocks to fit an SM (228 KB, 1 KB reserved
+  // per block).
+  constexpr int TWO_BLOCK_BYTES = (228 * 1024) / 2 - 1024;
+
+  // The layout a kernel uses.  RB = bytes per value (8 for FP64 and packed
+  // FP32).  More than 5 grains in 3D: in place where two blocks then fit an SM
+  // (FP32: three), with the next tile's boxes double-buffered if they fit too;
+  // not for the tensorial Jacobian product, which is bound by registers.  J v
+  // of 9 grains, scalar, at 96^3 cells: FP64 701 -> 602 us, FP32 500 -> 417 us.
+  template <int DIM, int G, bool TENS, bool JVP, bool HIST, bool ADV, int RB>
+  struct ThreePhasePlan
+  {
+    template <int NBUF>
+    using InPlace = ThreePhaseLayout<DIM, G, TENS, JVP, HIST, ADV, true, NBUF>;
+    static constexpr bool IN_PLACE =
+      DIM == 3 && G > 5 && !ADV && !(JVP && TENS) && InPlace<1>::TOTAL * RB <= TWO_BLOCK_BYTES;
+    static constexpr int  NBUF =
+      JVP && (!IN_PLACE || InPlace<2>::TOTAL * RB <= TWO_BLOCK_BYTES) ? 2 : 1;
+    using type = ThreePhaseLayout<DIM, G, TENS, JVP, HIST, ADV, IN_PLACE, NBUF>;
+  };
+  template <int DIM, int G, bool TENS, bool JVP, bool HIST, bool ADV, int RB>
+  using ThreePhaseSmem = typename ThreePhasePlan<DIM, G, TENS, JVP, HIST, ADV, RB>::type;
 
   // -------------------------------------------------------------------------
   // Jacobian-vector product: dst = J(lin) src.
@@ -681,18 +875,26 @@ namespace sint
   // of the next tile are copied (cp.async) into the second half of a double
   // buffer while the current tile is computed.
   // Two resident blocks per SM (<= 128 registers) unless the 3D FP64 grain
-  // state of large G would spill (one block, up to 255 registers); the light
-  // 2D FP32 product runs three (<= 85 registers), and the grain cut-off's
-  // G = 0 class (c and mu only) four (<= 64 registers).
-  template <int DIM, int G, typename R>
+  // state of large G would spill (one block, up to 255 registers; two where
+  // the point results are in place); the light 2D FP32 product runs three (<=
+  // 85 registers), and the grain cut-off's G = 0 class (c and mu only) four
+  // (<= 64 registers).
+  template <int DIM, int G, bool TENS, typename R, bool ADV>
   constexpr int jvp_blocks_per_sm()
   {
-    return G == 0 ? 4 : (DIM == 3 && sizeof(R) == 8 && G > 5) ? 1 : (DIM == 2 && sizeof(R) == 4) ? 3 : 2;
+    return G == 0                                                               ? 4 :
+           ThreePhasePlan<DIM, G, TENS, true, false, ADV, sizeof(R)>::IN_PLACE  ? (sizeof(R) == 4 ? 3 : 2) :
+           (DIM == 3 && sizeof(R) == 8 && G > 5)                                ? 1 :
+           (DIM == 2 && sizeof(R) == 4)                                         ? 3 :
+                                                                                  2;
   }
-  template <int DIM, int G>
+  template <int DIM, int G, bool TENS, bool HIST, bool ADV>
   constexpr int residual_blocks_per_sm()
   {
-    return G == 0 ? 4 : (DIM == 3 && G > 5) ? 1 : 2;
+    return G == 0                                                         ? 4 :
+           ThreePhasePlan<DIM, G, TENS, false, HIST, ADV, 8>::IN_PLACE    ? 2 :
+           (DIM == 3 && G > 5)                                            ? 1 :
+                                                                            2;
   }
 
   // CUT: grain cut-off.  The kernel instantiated for G grains runs over the
@@ -703,19 +905,21 @@ namespace sint
   // behind the current tile.
   // ADV: with the advection terms of the grains' rigid-body velocities.
   template <int DIM, int G, bool TENS, typename R, bool CUT, bool ADV = false>
-  __global__ void __launch_bounds__(Tile<DIM>::THREADS, jvp_blocks_per_sm<DIM, G, R>())
+  __global__ void __launch_bounds__(Tile<DIM>::THREADS, jvp_blocks_per_sm<DIM, G, TENS, R, ADV>())
     jvp_kernel(const Grid g, const Phys ph, const R *__restrict__ lin, const R *__restrict__ src,
                R *__restrict__ dst, R *__restrict__ partial, const CutTiles ct, const AdvData adv)
   {
     using T  = Tile<DIM>;
-    using SM = ThreePhaseSmem<DIM, G, TENS, true, false, ADV>;
-    constexpr int C = G + 2;
+    using SM = ThreePhaseSmem<DIM, G, TENS, true, false, ADV, sizeof(R)>;
+    using FM = typename SM::FM;
+    using PL = ThreePhasePlan<DIM, G, TENS, true, false, ADV, sizeof(R)>;
+    constexpr int C = G + 2, NBUF = SM::BUFFERS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R *s_buf = reinterpret_cast<R *>(smem_raw); // 2 x BOXES
-    R *F     = s_buf + 2 * SM::BOXES;
-    R *P     = F + SM::F_SIZE;
-    R *K     = F; // aliases the point fields, dead after phase 2
-    R *A_vel = P + SM::P_SIZE;
+    R *s_buf = reinterpret_cast<R *>(smem_raw); // NBUF x BOXES
+    R *F     = s_buf + NBUF * SM::BOXES;
+    R *P     = F + SM::P_AT;
+    R *K     = F + SM::K_AT;
+    R *A_vel = F + SM::F_SIZE + SM::P_SIZE;
     unsigned char *A_has = reinterpret_cast<unsigned char *>(A_vel + SM::ADV_VEL);
 
     const PhysR<R>           p(ph);
@@ -772,15 +976,15 @@ namespace sint
     for (int it = 0; idx < i1; ++it, idx += gridDim.x)
       {
         const long long nidx = idx + gridDim.x;
-        R              *nb   = s_buf + ((it + 1) & 1) * SM::BOXES;
+        R              *nb   = s_buf + (NBUF == 2 ? ((it + 1) & 1) * SM::BOXES : 0);
         long long       t_nn = 0; // the tile after next (CUT)
         unsigned long long gl_nn = 0;
         unsigned           tm_nn = 0;
+        const TileCoord    tcn = tile_coord_of<DIM>(g, CUT ? t_next : (nidx < i1 ? nidx : idx));
         if (nidx < i1)
           {
-            const long long next = CUT ? t_next : nidx;
-            const TileCoord tcn  = tile_coord_of<DIM>(g, next);
-            prefetch(nb, tcn, gl_next);
+            if constexpr (NBUF == 2)
+              prefetch(nb, tcn, gl_next);
             if constexpr (CUT)
               {
                 m_glob_next = cell_mask<DIM>(ct.cell_mask, g, tcn, cell);
@@ -792,34 +996,46 @@ namespace sint
                   }
               }
           }
-        cp_async_commit();
-        cp_async_wait<1>(); // this tile's group has landed (only the prefetch may be pending)
+        if constexpr (NBUF == 2)
+          {
+            cp_async_commit();
+            cp_async_wait<1>(); // this tile's group has landed (only the prefetch may be pending)
+          }
+        else
+          cp_async_wait<0>();
         __syncthreads();
         const TileCoord tc = tile_coord_of<DIM>(g, tile);
-        const R        *cb = s_buf + (it & 1) * SM::BOXES;
+        const R        *cb = s_buf + (NBUF == 2 ? (it & 1) * SM::BOXES : 0);
         const unsigned  m  = CUT ? local_mask<G>(m_glob, gl) : ~0u;
         if constexpr (ADV)
           adv_stage<DIM, G, R, CUT>(adv, g, tc, gl, A_vel, A_has);
-        phase_evaluate<DIM, G, TENS, true, false, R, CUT>(cb, cb + C * T::BOXS, F, k, m);
+        phase_evaluate<DIM, G, TENS, true, false, R, CUT, PL::IN_PLACE>(cb, cb + C * T::BOXS, F, k, m);
         __syncthreads();
-        jvp_point<DIM, G, TENS, R>(p, F, P, threadIdx.x / T::CELLS, cell, m);
+        jvp_point<DIM, G, TENS, FM, R>(p, F, P, threadIdx.x / T::CELLS, cell, m);
         if constexpr (ADV)
           {
-            using FM = FieldMap<DIM, G, TENS, true, false>;
             advect_c_point<DIM, G, R, CUT>(k, g, F, FM::base(FM::src_c), P, threadIdx.x / T::CELLS, cell, m, A_vel,
                                            A_has);
           }
         __syncthreads();
-        phase_integrate<DIM, G, R, CUT, ADV>(p, g, k, tc, P, cb + C * T::BOXS, K, m, A_vel, A_has);
+        phase_integrate<DIM, G, FM, R, CUT, ADV>(p, g, k, tc, P, cb + C * T::BOXS, K, m, A_vel, A_has);
         __syncthreads();
+        if constexpr (NBUF == 1)
+          {
+            // one box buffer: its last readers have passed, the next tile's
+            // copies run behind the stores below
+            if (nidx < i1)
+              prefetch(nb, tcn, gl_next);
+            cp_async_commit();
+          }
         if (tile_interior<DIM>(g, tc))
           sum_and_store_interior<DIM>(K, C, g, tc.linear, np, tile_node0(g, tc), dst, partial, gl, CUT, ct.c_all, tm);
         else
           sum_and_store<DIM>(K, C, g, tc, BoxNode<DIM>(g, tc), dst, partial, gl, CUT, ct.c_all, tm);
-        // No further barrier: the next tile's prefetch writes the other box
-        // buffer, whose last readers (this tile's phases 1 and 3) passed the
-        // barrier after phase 3, and K (aliasing F) is next written in phase
-        // 1, after the barrier that follows the next cp.async wait.
+        // No further barrier: the next tile's prefetch writes a box buffer whose
+        // last readers (phases 1 and 3) have passed the barrier after phase 3,
+        // and K (inside F) is next written in phase 1, after the barrier that
+        // follows the next cp.async wait.
         if constexpr (CUT)
           {
             tile    = t_next;
@@ -837,7 +1053,7 @@ namespace sint
   }
 
   // -------------------------------------------------------------------------
-  // FP32 Jacobian-vector product on tile pairs.  sm_100 executes FP32 add,
+  // FP32 Jacobian-vector product of few grains on tile pairs.  sm_100 executes FP32 add,
   // multiply and fused multiply-add on two values held in a 64-bit register
   // pair with one instruction (FADD2 / FMUL2 / FFMA2); the FP32 product is
   // bound by instruction issue, so the block computes tiles 2j and 2j + 1
@@ -853,26 +1069,28 @@ namespace sint
   // Resident blocks per SM: as the FP64 product (pairs take the FP64 product's
   // registers), but three for the class without grains, whose pairs need
   // ~70 registers (four blocks would cap them at 64 and spill).
-  template <int DIM, int G>
+  template <int DIM, int G, bool TENS>
   constexpr int jvp_pair_blocks_per_sm()
   {
-    return G == 0 ? 3 : jvp_blocks_per_sm<DIM, G, double>();
+    return G == 0 ? 3 : jvp_blocks_per_sm<DIM, G, TENS, double, false>();
   }
 
   template <int DIM, int G, bool TENS, bool CUT = false>
-  __global__ void __launch_bounds__(Tile<DIM>::THREADS, jvp_pair_blocks_per_sm<DIM, G>())
+  __global__ void __launch_bounds__(Tile<DIM>::THREADS, jvp_pair_blocks_per_sm<DIM, G, TENS>())
     jvp_pair_kernel(const Grid g, const Phys ph, const float *__restrict__ lin, const float *__restrict__ src,
                     float *__restrict__ dst, float *__restrict__ partial, const CutTiles ct)
   {
     static_assert(!CUT || G == 0, "the cut-off pair kernel serves the class without grains");
     using T  = Tile<DIM>;
-    using SM = ThreePhaseSmem<DIM, G, TENS, true, false, false>;
+    using SM = ThreePhaseSmem<DIM, G, TENS, true, false, false, sizeof(F2)>;
+    using FM = typename SM::FM;
+    static_assert(G <= 4 && SM::BUFFERS == 2, "pairs serve few grains");
     constexpr int C = G + 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     F2 *s_buf = reinterpret_cast<F2 *>(smem_raw); // 2 x BOXES pairs
     F2 *F     = s_buf + 2 * SM::BOXES;
-    F2 *P     = F + SM::F_SIZE;
-    F2 *K     = F; // aliases the point fields, dead after phase 2
+    F2 *P     = F + SM::P_AT;
+    F2 *K     = F + SM::K_AT;
 
     const PhysR<F2>           p(ph);
     const CellConsts<DIM, F2> k(g);
@@ -927,9 +1145,9 @@ namespace sint
         const F2       *cb     = s_buf + (it & 1) * SM::BOXES;
         phase_evaluate<DIM, G, TENS, true, false, F2, false>(cb, cb + C * T::BOXS, F, k);
         __syncthreads();
-        jvp_point<DIM, G, TENS, F2>(p, F, P, threadIdx.x / T::CELLS, cell);
+        jvp_point<DIM, G, TENS, FM, F2>(p, F, P, threadIdx.x / T::CELLS, cell);
         __syncthreads();
-        phase_integrate<DIM, G, F2, false, false>(p, g, k, tca, P, cb + C * T::BOXS, K, ~0u, nullptr, nullptr,
+        phase_integrate<DIM, G, FM, F2, false, false>(p, g, k, tca, P, cb + C * T::BOXS, K, ~0u, nullptr, nullptr,
                                                   &tcb);
         __syncthreads();
 #pragma unroll
@@ -960,22 +1178,24 @@ namespace sint
   // compacted components, as the Jacobian product does.
   // ADV: with the advection terms of the grains' rigid-body velocities.
   template <int DIM, int G, bool TENS, int WTD, bool CUT, bool ADV = false>
-  __global__ void __launch_bounds__(Tile<DIM>::THREADS, residual_blocks_per_sm<DIM, G>())
+  __global__ void __launch_bounds__(Tile<DIM>::THREADS, residual_blocks_per_sm<DIM, G, TENS, WTD == 2, ADV>())
     residual_kernel(const Grid g, const Phys ph, const double *__restrict__ src, const double *__restrict__ h0,
                     const double *__restrict__ h1, const double *__restrict__ h2, double *__restrict__ dst,
                     double *__restrict__ partial, const CutTiles ct, const AdvData adv)
   {
     using R  = double;
     using T  = Tile<DIM>;
-    using SM = ThreePhaseSmem<DIM, G, TENS, false, WTD == 2, ADV>;
+    using SM = ThreePhaseSmem<DIM, G, TENS, false, WTD == 2, ADV, sizeof(double)>;
+    using FM = typename SM::FM;
+    using PL = ThreePhasePlan<DIM, G, TENS, false, WTD == 2, ADV, sizeof(double)>;
     constexpr int C = G + 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *s_u = reinterpret_cast<R *>(smem_raw);
     R *s_h = s_u + C * T::BOXS;
     R *F   = s_u + SM::BOXES;
-    R *P   = F + SM::F_SIZE;
-    R *K   = F;
-    R *A_vel = P + SM::P_SIZE;
+    R *P   = F + SM::P_AT;
+    R *K   = F + SM::K_AT;
+    R *A_vel = F + SM::F_SIZE + SM::P_SIZE;
     unsigned char *A_has = reinterpret_cast<unsigned char *>(A_vel + SM::ADV_VEL);
 
     const PhysR<R>           p(ph);
@@ -1028,17 +1248,19 @@ namespace sint
         if constexpr (ADV)
           adv_stage<DIM, G, R, CUT>(adv, g, tc, gl, A_vel, A_has);
         __syncthreads();
-        phase_evaluate<DIM, G, TENS, false, WTD == 2, R, CUT>(s_u, s_h, F, k, m);
+        phase_evaluate<DIM, G, TENS, false, WTD == 2, R, CUT, PL::IN_PLACE>(s_u, s_h, F, k, m);
         __syncthreads();
-        residual_point<DIM, G, TENS, WTD, R>(p, F, P, threadIdx.x / T::CELLS, threadIdx.x % T::CELLS, m);
+        if constexpr (PL::IN_PLACE)
+          residual_point_streamed<DIM, G, TENS, WTD, FM, R>(p, F, threadIdx.x / T::CELLS, threadIdx.x % T::CELLS, m);
+        else
+          residual_point<DIM, G, TENS, WTD, FM, R>(p, F, P, threadIdx.x / T::CELLS, threadIdx.x % T::CELLS, m);
         if constexpr (ADV)
           {
-            using FM = FieldMap<DIM, G, TENS, false, WTD == 2>;
             advect_c_point<DIM, G, R, CUT>(k, g, F, FM::base(FM::lin_c), P, threadIdx.x / T::CELLS,
                                            threadIdx.x % T::CELLS, m, A_vel, A_has);
           }
         __syncthreads();
-        phase_integrate<DIM, G, R, CUT, ADV>(p, g, k, tc, P, s_u, K, m, A_vel, A_has);
+        phase_integrate<DIM, G, FM, R, CUT, ADV>(p, g, k, tc, P, s_u, K, m, A_vel, A_has);
         __syncthreads();
         if (interior)
           sum_and_store_interior<DIM>(K, C, g, tc.linear, np, node0, dst, partial, gl, CUT, ct.c_all, tm, &ph.hooks);

@@ -54,12 +54,12 @@ namespace sint
   cudaError_t launch_jvp_g(const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
                            const CutTiles &ct, const AdvData &adv, cudaStream_t s)
   {
-    const size_t smem = ThreePhaseSmem<DIM, G, TENS, true, false, ADV>::TOTAL * sizeof(R);
+    const size_t smem = ThreePhaseSmem<DIM, G, TENS, true, false, ADV, sizeof(R)>::TOTAL * sizeof(R);
     auto         k    = jvp_kernel<DIM, G, TENS, R, CUT, ADV>;
     static DeviceCache cache;
     int                grid_cap = 0;
     if (const cudaError_t e =
-          persistent_grid(cache, k, smem, jvp_blocks_per_sm<DIM, G, R>(), Tile<DIM>::THREADS, grid_cap))
+          persistent_grid(cache, k, smem, jvp_blocks_per_sm<DIM, G, TENS, R, ADV>(), Tile<DIM>::THREADS, grid_cap))
       return e;
     const long long blocks = g.n_tiles < grid_cap ? g.n_tiles : grid_cap;
     k<<<dim3((unsigned)blocks), Tile<DIM>::THREADS, smem, s>>>(g, p, lin, src, dst, partial, ct, adv);
@@ -71,12 +71,12 @@ namespace sint
   cudaError_t launch_jvp_pair_g(const Grid &g, const Phys &p, const float *lin, const float *src, float *dst,
                                 float *partial, cudaStream_t s, const CutTiles &ct = CutTiles())
   {
-    const size_t smem = ThreePhaseSmem<DIM, G, TENS, true, false, false>::TOTAL * sizeof(F2);
+    const size_t smem = ThreePhaseSmem<DIM, G, TENS, true, false, false, sizeof(F2)>::TOTAL * sizeof(F2);
     auto         k    = jvp_pair_kernel<DIM, G, TENS, CUT>;
     static DeviceCache cache;
     int                grid_cap = 0;
     if (const cudaError_t e =
-          persistent_grid(cache, k, smem, jvp_pair_blocks_per_sm<DIM, G>(), Tile<DIM>::THREADS, grid_cap))
+          persistent_grid(cache, k, smem, jvp_pair_blocks_per_sm<DIM, G, TENS>(), Tile<DIM>::THREADS, grid_cap))
       return e;
     // the class size of the cut-off lives on the device: a full persistent grid
     const long long pairs  = CUT ? (long long)grid_cap : (g.n_tiles + 1) / 2;
@@ -91,12 +91,12 @@ namespace sint
                                 double *dst, double *partial, const CutTiles &ct, const AdvData &adv,
                                 cudaStream_t s)
   {
-    const size_t  smem     = ThreePhaseSmem<DIM, G, TENS, false, WTD == 2, ADV>::TOTAL * sizeof(double);
+    const size_t  smem     = ThreePhaseSmem<DIM, G, TENS, false, WTD == 2, ADV, sizeof(double)>::TOTAL * sizeof(double);
     auto          k        = residual_kernel<DIM, G, TENS, WTD, CUT, ADV>;
     static DeviceCache cache;
     int                grid_cap = 0;
     if (const cudaError_t e =
-          persistent_grid(cache, k, smem, residual_blocks_per_sm<DIM, G>(), Tile<DIM>::THREADS, grid_cap))
+          persistent_grid(cache, k, smem, residual_blocks_per_sm<DIM, G, TENS, WTD == 2, ADV>(), Tile<DIM>::THREADS, grid_cap))
       return e;
     const double *h0     = WTD == 2 ? hist[0] : nullptr;
     const double *h1     = (WTD == 2 && p.order > 1) ? hist[1] : nullptr;
@@ -216,15 +216,20 @@ namespace sint
 #undef SINT_CALL
   }
 
-  // The full operator's J v: one kernel in 2D (sint_fused2d.cuh), packed FP32
-  // tile pairs, or the tiled kernel.
+  // The full operator's J v: one kernel in 2D (sint_fused2d.cuh), in 3D packed
+  // FP32 tile pairs for few grains, or the tiled kernel.  Pairs take 8 bytes
+  // per value: with more grains one block fits an SM's registers, and the
+  // scalar FP32 kernel with two (tensorial) or three (scalar mobility) is
+  // faster (160^3 cells: 9 grains tensorial 3347 us on pairs, 2967 us here; 5
+  // grains 1700 / 1647 us, 4 grains 1367 / 1380 us; scalar mobility, 9 grains
+  // 2216 / 1816 us, 5 grains 1264 / 1254 us, 4 grains 1105 / 1116 us).
   template <int DIM, int G, bool TENS, typename R, bool ADV>
   cudaError_t launch_jvp_full(const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
                               const AdvData &adv, cudaStream_t s)
   {
     if constexpr (!ADV && runs_fused2d(DIM, G, TENS, sizeof(R)))
       return launch_fused2d_g<G, TENS, R, -1>(g, p, Fused2DArgs<R>{lin, src, {}, dst, 0}, s);
-    else if constexpr (!ADV && std::is_same_v<R, float>)
+    else if constexpr (!ADV && std::is_same_v<R, float> && G <= 4)
       return launch_jvp_pair_g<DIM, G, TENS>(g, p, lin, src, dst, partial, s);
     else
       return launch_jvp_g<DIM, G, TENS, R, false, ADV>(g, p, lin, src, dst, partial, CutTiles(), adv, s);
