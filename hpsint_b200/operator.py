@@ -93,12 +93,16 @@ def bdf_weights(order, dt):
     return w
 
 
+# A product of a small mesh is shorter on the GPU than its call: pointers go to
+# the library as plain integers (its argument types are declared) and the
+# current stream is read as a handle, without a Stream object (FP64 J v of 256 x
+# 128 cells, call after call: 9.0 -> 5.9 us).
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 class SinteringOperatorGeneric:
@@ -118,6 +122,7 @@ class SinteringOperatorGeneric:
         n, c, ld = ctypes.c_int64(), ctypes.c_int(), ctypes.c_int64()
         L.check(lib.sint_dof_layout(self._h, ctypes.byref(n), ctypes.byref(c), ctypes.byref(ld)), "sint_dof_layout")
         self.N, self.C, self.ld = n.value, c.value, ld.value
+        self._numel = self.C * self.ld
         self.order = 0
         self.cut_off_tolerance = 0.0
 
@@ -337,14 +342,17 @@ class SinteringOperatorGeneric:
                                                 ctypes.byref(hooks), _stream()), "sint_residual_f64_hooks")
 
     def vmult(self, dst, src):
-        if src.dtype == torch.float32:
-            self._check_vec(dst, torch.float32)
-            self._check_vec(src, torch.float32)
-            L.check(L.lib().sint_jvp_f32(self._h, _ptr(dst), _ptr(src), _stream()), "sint_jvp_f32")
+        dtype = src.dtype
+        if dtype is not torch.float32:
+            dtype = torch.float64
+        self._check_vec(dst, dtype)
+        self._check_vec(src, dtype)
+        if dtype is torch.float32:
+            status = L.lib().sint_jvp_f32(self._h, dst.data_ptr(), src.data_ptr(), _stream())
         else:
-            self._check_vec(dst, torch.float64)
-            self._check_vec(src, torch.float64)
-            L.check(L.lib().sint_jvp_f64(self._h, _ptr(dst), _ptr(src), _stream()), "sint_jvp_f64")
+            status = L.lib().sint_jvp_f64(self._h, dst.data_ptr(), src.data_ptr(), _stream())
+        if status:
+            L.check(status, "sint_jvp_f32" if dtype is torch.float32 else "sint_jvp_f64")
 
     def do_update(self):
         pass
@@ -361,7 +369,7 @@ class SinteringOperatorGeneric:
 
     # --- helpers --------------------------------------------------------------
     def _check_vec(self, t, dtype):
-        if not (t.is_cuda and t.dtype == dtype and t.is_contiguous() and t.numel() == self.C * self.ld):
+        if not (t.is_cuda and t.dtype is dtype and t.is_contiguous() and t.numel() == self._numel):
             raise ValueError(f"expected a contiguous CUDA {dtype} block vector of shape ({self.C}, {self.ld})")
 
     def to_device(self, arr_cn, dtype=torch.float64):
