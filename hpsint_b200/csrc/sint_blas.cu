@@ -3,6 +3,7 @@
 // Reductions are deterministic: a fixed grid of NB_RED blocks writes block
 // partials in FP64, one block sums them in a fixed tree order.
 #include <string>
+#include <type_traits>
 
 #include "sint_internal.h"
 #include "sint_launch.h"
@@ -113,11 +114,12 @@ namespace sint
   }
 
   // Fused finish of a reduction: every block has written its partials
-  // (rows 0..m-1, NB_RED blocks each); the block that takes the last ticket
-  // sums each row in a fixed order (lane l adds blocks l, l + 32, ..., then a
-  // fixed butterfly), writes out[0..m) and resets the ticket.  The result does
-  // not depend on which block finishes last.
-  __device__ __forceinline__ void finish_if_last(const double *__restrict__ rows, int m, double *__restrict__ out,
+  // (rows 0..m-1, one column per block, row pitch NB_RED); the block that
+  // takes the last ticket sums each row in a fixed order (lane l adds blocks
+  // l, l + 32, ..., then a fixed butterfly), writes out[0..m) and resets the
+  // ticket.  The result does not depend on which block finishes last.  Returns
+  // whether this is that block.
+  __device__ __forceinline__ bool finish_if_last(const double *__restrict__ rows, int m, double *__restrict__ out,
                                                  unsigned *ticket)
   {
     __shared__ bool last;
@@ -127,20 +129,36 @@ namespace sint
       last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last)
-      return;
+      return false;
     __threadfence();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = gridDim.x;
     for (int j = warp; j < m; j += RED_THREADS / 32)
       {
+        // a row's loads are all in flight together
+        constexpr int L = (NB_RED + 31) / 32;
+        double        t[L];
+#pragma unroll
+        for (int i = 0; i < L; ++i)
+          t[i] = lane + 32 * i < nb ? __ldcg(rows + (size_t)j * NB_RED + lane + 32 * i) : 0.0;
         double v = 0.0;
-        for (int b = lane; b < NB_RED; b += 32)
-          v += __ldcg(rows + (size_t)j * NB_RED + b);
+#pragma unroll
+        for (int i = 0; i < L; ++i)
+          v += t[i];
         v = warp_sum(v);
         if (lane == 0)
           out[j] = v;
       }
     if (threadIdx.x == 0)
       *ticket = 0u;
+    return true;
+  }
+
+  // Blocks of a reduction over nc packs: one pack per thread until NB_RED
+  // blocks are reached (a 2D Krylov vector of 130,000 values fills 260).
+  static unsigned red_blocks(long long nc)
+  {
+    const long long b = (nc + RED_THREADS - 1) / RED_THREADS;
+    return (unsigned)(b < 1 ? 1 : (b < NB_RED ? b : NB_RED));
   }
 
   // partial[j * NB_RED + blockIdx.x] = sum over this block's chunks of w . V_j
@@ -151,14 +169,16 @@ namespace sint
                     double *__restrict__ partial, const int *__restrict__ cond, const double *__restrict__ rows,
                     int m_total, double *__restrict__ out, unsigned *ticket, const uint32_t *__restrict__ live)
   {
+    dependent_start();
     if (cond && *cond == 0)
       return;
-    __shared__ double s_w[RED_THREADS / 32];
+    constexpr int     NW = RED_THREADS / 32;
+    __shared__ double s_w[M][NW];
     double            acc[M];
 #pragma unroll
     for (int j = 0; j < M; ++j)
       acc[j] = 0.0;
-    for (long long c = (long long)blockIdx.x * RED_THREADS + threadIdx.x; c < nc; c += (long long)NB_RED * RED_THREADS)
+    for (long long c = (long long)blockIdx.x * RED_THREADS + threadIdx.x; c < nc; c += (long long)gridDim.x * RED_THREADS)
       {
         if (!chunk_live(live, c * E))
           continue;
@@ -173,19 +193,38 @@ namespace sint
                 acc[j] += double(wi.v[e]) * double(vj.v[e]);
             }
       }
+    // all rows through the warps at once: one barrier for the block
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
     for (int j = 0; j < M; ++j)
       if (j < m)
         {
-          const double s = block_sum(acc[j], s_w);
-          if (threadIdx.x == 0)
-            partial[j * NB_RED + blockIdx.x] = s;
+          const double v = warp_sum(acc[j]);
+          if (lane == 0)
+            s_w[j][wid] = v;
         }
+    __syncthreads();
+    for (int j = threadIdx.x; j < m; j += RED_THREADS)
+      {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k)
+          v += s_w[j][k];
+        partial[(size_t)j * NB_RED + blockIdx.x] = v;
+      }
     if (out)
       finish_if_last(rows, m_total, out, ticket);
   }
 
-  constexpr int MD = 16; // vectors per multidot / multiaxpy pass (accumulators in registers)
+  // Vectors per multidot / multiaxpy pass, and the instances for few vectors
+  // (an instance tests each of its M vectors against m).
+  constexpr int MD = 16;
+  template <typename F>
+  static cudaError_t by_count(int m, F go)
+  {
+    return m <= 4 ? go(std::integral_constant<int, 4>{}) :
+           m <= 8 ? go(std::integral_constant<int, 8>{}) : go(std::integral_constant<int, MD>{});
+  }
 
   template <typename R>
   static int launch_multidot(Ctx *c, long long n, const R *w, const R *V, long long stride, int m, double *out,
@@ -196,23 +235,25 @@ namespace sint
         set_error("multidot: m out of range");
         return SINT_ERR_ARG;
       }
-    constexpr int E    = pack_of<R>();
-    const bool    pack = can_pack<R>(n, stride, w, V);
+    constexpr int  E    = pack_of<R>();
+    const bool     pack = can_pack<R>(n, stride, w, V);
+    const unsigned nb   = red_blocks(pack ? n / E : n); // the same for every pass: the last one sums all rows
     for (int j0 = 0; j0 < m; j0 += MD)
       {
-        const int mm   = m - j0 < MD ? m - j0 : MD;
-        double   *pp   = c->red + (size_t)j0 * NB_RED;
-        double   *outl = j0 + MD >= m ? out : nullptr; // the last pass sums all rows
-        if (pack)
-          multidot_kernel<R, MD, E><<<NB_RED, RED_THREADS, 0, s>>>(n / E, w, V + j0 * stride, stride, mm, pp, cond,
-                                                                   c->red, m, outl, c->red_ticket, live);
-        else
-          multidot_kernel<R, MD, 1><<<NB_RED, RED_THREADS, 0, s>>>(n, w, V + j0 * stride, stride, mm, pp, cond,
-                                                                   c->red, m, outl, c->red_ticket, live);
-        count_launches(1);
+        const int         mm   = m - j0 < MD ? m - j0 : MD;
+        double           *pp   = c->red + (size_t)j0 * NB_RED;
+        double           *outl = j0 + MD >= m ? out : nullptr;
+        const cudaError_t e    = by_count(mm, [&](auto k) {
+          constexpr int M = decltype(k)::value;
+          return pack ? launch_dependent(multidot_kernel<R, M, E>, nb, RED_THREADS, 0, s, n / E, w, V + j0 * stride,
+                                            stride, mm, pp, cond, c->red, m, outl, c->red_ticket, live) :
+                           launch_dependent(multidot_kernel<R, M, 1>, nb, RED_THREADS, 0, s, n, w, V + j0 * stride,
+                                            stride, mm, pp, cond, c->red, m, outl, c->red_ticket, live);
+        });
+        if (e != cudaSuccess)
+          return cuda_fail(e, "multidot");
       }
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? SINT_OK : cuda_fail(e, "multidot");
+    return SINT_OK;
   }
 
   template <typename R>
@@ -247,13 +288,21 @@ namespace sint
   }
 
   // w -= sum_j coef[j] V_j (j < m <= M); with `partial`, also the block
-  // partials of |w|^2 after the update (FP64), for the norm that follows.
+  // partials of |w|^2 after the update (FP64), for the norm that follows, and
+  // with chk.H the bookkeeping of an Arnoldi step after its first
+  // Gram-Schmidt pass (in the block that finishes the norm): Hessenberg column
+  // j = h and deal.II's re-orthogonalisation test (Kelley 1995, as in
+  // SolverGMRES): once |w| after the pass falls below 10 sqrt(eps) of |w|
+  // before it, every later iteration of this solve takes a second pass (the
+  // flag is sticky).  thresh2 = 100 eps of the Krylov vectors' precision;
+  // |w|^2 before = |h|^2 + |w'|^2.
   template <typename R, int M, int E>
   __global__ void __launch_bounds__(RED_THREADS)
     multiaxpy_kernel(long long nc, R *__restrict__ w, const R *__restrict__ V, long long stride, int m,
                      const double *__restrict__ coef, double *__restrict__ partial, const int *__restrict__ cond,
-                     double *__restrict__ norm2_out, unsigned *ticket, const uint32_t *__restrict__ live)
+                     double *norm2_out, unsigned *ticket, const uint32_t *__restrict__ live, const ArnoldiCheck chk)
   {
+    dependent_start();
     if (cond && *cond == 0)
       return;
     __shared__ R      s_c[M];
@@ -289,32 +338,51 @@ namespace sint
         const double t = block_sum(nrm, s_w);
         if (threadIdx.x == 0)
           partial[blockIdx.x] = t;
-        finish_if_last(partial, 1, norm2_out, ticket);
+        if (!finish_if_last(partial, 1, norm2_out, ticket) || !chk.H || threadIdx.x >= 32)
+          return;
+        double *hcol = chk.H + (long long)chk.j * chk.ldh;
+        double  hh   = 0.0;
+        for (int i = threadIdx.x; i <= chk.j; i += 32)
+          {
+            const double h = chk.d_s[i];
+            hcol[i]        = h;
+            hh += h * h;
+          }
+        hh = warp_sum(hh);
+        __syncwarp();
+        if (threadIdx.x == 0)
+          {
+            const double nw2 = *norm2_out; // written by this thread in finish_if_last
+            if (nw2 < chk.thresh2 * (hh + nw2))
+              *chk.reorth = 1;
+          }
       }
   }
 
   template <typename R>
   static int launch_multiaxpy(Ctx *c, long long n, R *w, const R *V, long long stride, int m, const double *coef,
                               double *norm2_out, cudaStream_t s, const int *cond = nullptr,
-                              const uint32_t *live = nullptr)
+                              const uint32_t *live = nullptr, const ArnoldiCheck &chk = ArnoldiCheck())
   {
-    constexpr int E    = pack_of<R>();
-    const bool    pack = can_pack<R>(n, stride, w, V);
+    constexpr int  E    = pack_of<R>();
+    const bool     pack = can_pack<R>(n, stride, w, V);
+    const unsigned nb   = red_blocks(pack ? n / E : n);
     for (int j0 = 0; j0 < m; j0 += MD)
       {
-        const int mm   = m - j0 < MD ? m - j0 : MD;
-        double   *part = (norm2_out && j0 + MD >= m) ? c->red : nullptr; // norm in the last pass
-        unsigned *tk   = c ? c->red_ticket : nullptr;
-        if (pack)
-          multiaxpy_kernel<R, MD, E><<<NB_RED, RED_THREADS, 0, s>>>(n / E, w, V + j0 * stride, stride, mm, coef + j0,
-                                                                    part, cond, norm2_out, tk, live);
-        else
-          multiaxpy_kernel<R, MD, 1><<<NB_RED, RED_THREADS, 0, s>>>(n, w, V + j0 * stride, stride, mm, coef + j0,
-                                                                    part, cond, norm2_out, tk, live);
-        count_launches(1);
+        const int         mm   = m - j0 < MD ? m - j0 : MD;
+        double           *part = (norm2_out && j0 + MD >= m) ? c->red : nullptr; // norm in the last pass
+        unsigned         *tk   = c ? c->red_ticket : nullptr;
+        const cudaError_t e    = by_count(mm, [&](auto k) {
+          constexpr int M = decltype(k)::value;
+          return pack ? launch_dependent(multiaxpy_kernel<R, M, E>, nb, RED_THREADS, 0, s, n / E, w, V + j0 * stride,
+                                            stride, mm, coef + j0, part, cond, norm2_out, tk, live, chk) :
+                           launch_dependent(multiaxpy_kernel<R, M, 1>, nb, RED_THREADS, 0, s, n, w, V + j0 * stride,
+                                            stride, mm, coef + j0, part, cond, norm2_out, tk, live, chk);
+        });
+        if (e != cudaSuccess)
+          return cuda_fail(e, "multiaxpy");
       }
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? SINT_OK : cuda_fail(e, "multiaxpy");
+    return SINT_OK;
   }
 
   template <typename R>
@@ -327,14 +395,14 @@ namespace sint
 
   template <typename R>
   int multiaxpy_norm2(Ctx *c, long long n, R *w, const R *V, long long stride, int m, const double *coef,
-                      double *norm2_out, cudaStream_t s, const uint32_t *live)
+                      double *norm2_out, cudaStream_t s, const uint32_t *live, const ArnoldiCheck &chk)
   {
-    return launch_multiaxpy<R>(c, n, w, V, stride, m, coef, norm2_out, s, nullptr, live);
+    return launch_multiaxpy<R>(c, n, w, V, stride, m, coef, norm2_out, s, nullptr, live, chk);
   }
   template int multiaxpy_norm2<double>(Ctx *, long long, double *, const double *, long long, int, const double *,
-                                       double *, cudaStream_t, const uint32_t *);
+                                       double *, cudaStream_t, const uint32_t *, const ArnoldiCheck &);
   template int multiaxpy_norm2<float>(Ctx *, long long, float *, const float *, long long, int, const double *,
-                                      double *, cudaStream_t, const uint32_t *);
+                                      double *, cudaStream_t, const uint32_t *, const ArnoldiCheck &);
 
   template <typename R>
   int multiaxpy_norm2_if(Ctx *c, long long n, R *w, const R *V, long long stride, int m, const double *coef,
@@ -399,14 +467,12 @@ namespace sint
                               const uint32_t *);
 
   // y = b y + a x; a term whose factor is 0 is dropped, so NaN in an unused
-  // operand does not spread.  With d_div: a = 1 / d_div[0] read on the device.
-  // Chunks that are not live are written as zero without reading.
+  // operand does not spread.  Chunks that are not live are written as zero
+  // without reading.
   template <typename R, int E>
-  __global__ void axpby_kernel(long long nc, R a, const R *__restrict__ x, R b, R *__restrict__ y,
-                               const double *__restrict__ d_div, const uint32_t *__restrict__ live)
+  __device__ __forceinline__ void axpby_body(long long nc, R a, const R *__restrict__ x, R b, R *__restrict__ y,
+                                             const uint32_t *__restrict__ live)
   {
-    if (d_div)
-      a = R(1.0 / d_div[0]);
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += (long long)gridDim.x * blockDim.x)
       {
         if (!chunk_live(live, c * E))
@@ -426,37 +492,115 @@ namespace sint
       }
   }
 
-  template <typename R>
-  static int launch_axpby(long long n, double a, const R *x, double b, R *y, const double *d_div, cudaStream_t s,
-                          const uint32_t *live = nullptr)
+  // Blocks of an element-wise pass of 256 threads over nc packs.
+  static unsigned map_blocks(long long nc)
   {
-    constexpr int E = pack_of<R>();
-    if (can_pack<R>(n, 0, x, y))
-      axpby_kernel<R, E><<<1184, 256, 0, s>>>(n / E, R(a), x, R(b), y, d_div, live);
-    else
-      axpby_kernel<R, 1><<<1184, 256, 0, s>>>(n, R(a), x, R(b), y, d_div, live);
-    count_launches(1);
-    const cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? SINT_OK : cuda_fail(e, "axpby");
+    const long long b = (nc + 255) / 256;
+    return (unsigned)(b < 1 ? 1 : (b < 1184 ? b : 1184));
+  }
+
+  template <typename R, int E>
+  __global__ void __launch_bounds__(256) axpby_kernel(long long nc, R a, const R *__restrict__ x, R b,
+                                                      R *__restrict__ y, const uint32_t *__restrict__ live)
+  {
+    dependent_start();
+    axpby_body<R, E>(nc, a, x, b, y, live);
   }
 
   template <typename R>
   int axpby(long long n, double a, const R *x, double b, R *y, cudaStream_t s, const uint32_t *live)
   {
-    return launch_axpby<R>(n, a, x, b, y, nullptr, s, live);
+    constexpr int     E = pack_of<R>();
+    const cudaError_t e =
+      can_pack<R>(n, 0, x, y) ?
+        launch_dependent(axpby_kernel<R, E>, map_blocks(n / E), 256, 0, s, n / E, R(a), x, R(b), y, live) :
+        launch_dependent(axpby_kernel<R, 1>, map_blocks(n), 256, 0, s, n, R(a), x, R(b), y, live);
+    return e == cudaSuccess ? SINT_OK : cuda_fail(e, "axpby");
   }
   template int axpby<double>(long long, double, const double *, double, double *, cudaStream_t, const uint32_t *);
   template int axpby<float>(long long, double, const float *, double, float *, cudaStream_t, const uint32_t *);
 
-  template <typename R>
-  int scale_by_device(long long n, const R *x, const double *d_div, R *y, cudaStream_t s, const uint32_t *live)
+  // End of Arnoldi step j after the (optional) second Gram-Schmidt pass: the
+  // next basis vector y = w / |w| by all blocks, and in block 0 the
+  // bookkeeping of the step: Hessenberg column, Givens rotations, residual
+  // estimate.  out[j] = {|g_{j+1}|, status}: 0 continue, 1 converged, 2
+  // breakdown, 3 non-finite.
+  template <typename R, int E>
+  __global__ void __launch_bounds__(256)
+    arnoldi_next_kernel(long long nc, const R *__restrict__ w, R *__restrict__ y, const uint32_t *__restrict__ live,
+                        const ArnoldiNext st)
   {
-    return launch_axpby<R>(n, 1.0, x, 0.0, y, d_div, s, live);
+    dependent_start();
+    const double nw = sqrt(fmax(st.d_s[MAX_MULTIDOT], 0.0));
+    if (blockIdx.x == 0)
+      {
+        // the column and the rotations in shared memory: the recurrence below
+        // is serial, its loads need not be
+        __shared__ double s_h[MAX_MULTIDOT + 1], s_c[MAX_MULTIDOT], s_s[MAX_MULTIDOT];
+        const int         j    = st.j;
+        double           *hcol = st.H + (long long)j * st.ldh;
+        if (int(threadIdx.x) <= j)
+          {
+            s_h[threadIdx.x] = hcol[threadIdx.x] + (*st.reorth ? st.d_s[threadIdx.x] : 0.0);
+            if (int(threadIdx.x) < j)
+              {
+                s_c[threadIdx.x] = st.cs[threadIdx.x];
+                s_s[threadIdx.x] = st.sn[threadIdx.x];
+              }
+          }
+        __syncthreads();
+        if (threadIdx.x == 0)
+          {
+            double a = s_h[0];
+            for (int i = 0; i < j; ++i)
+              {
+                const double b = s_h[i + 1];
+                s_h[i]         = s_c[i] * a + s_s[i] * b;
+                a              = -s_s[i] * a + s_c[i] * b;
+              }
+            const double rr = hypot(a, nw);
+            const double cj = rr == 0.0 ? 1.0 : a / rr, sj = rr == 0.0 ? 0.0 : nw / rr;
+            s_h[j]          = rr;
+            st.cs[j]        = cj;
+            st.sn[j]        = sj;
+            const double gj = st.g[j];
+            st.g[j + 1]     = -sj * gj;
+            st.g[j]         = cj * gj;
+            const double res = fabs(sj * gj);
+            double       status;
+            if (!isfinite(res) || !isfinite(nw))
+              status = 3.0;
+            else if (res <= *st.tol)
+              status = 1.0;
+            else if (nw == 0.0)
+              status = 2.0;
+            else
+              status = 0.0;
+            st.out[j] = make_double2(res, status);
+          }
+        __syncthreads();
+        if (int(threadIdx.x) <= j)
+          hcol[threadIdx.x] = s_h[threadIdx.x];
+        if (int(threadIdx.x) == j + 1)
+          hcol[j + 1] = 0.0;
+      }
+    axpby_body<R, E>(nc, R(1.0 / nw), w, R(0), y, live);
   }
-  template int scale_by_device<double>(long long, const double *, const double *, double *, cudaStream_t,
-                                       const uint32_t *);
-  template int scale_by_device<float>(long long, const float *, const double *, float *, cudaStream_t,
-                                      const uint32_t *);
+
+  template <typename R>
+  int arnoldi_next(long long n, const R *w, R *y, const ArnoldiNext &st, cudaStream_t s, const uint32_t *live)
+  {
+    constexpr int     E = pack_of<R>();
+    const cudaError_t e =
+      can_pack<R>(n, 0, w, y) ?
+        launch_dependent(arnoldi_next_kernel<R, E>, map_blocks(n / E), 256, 0, s, n / E, w, y, live, st) :
+        launch_dependent(arnoldi_next_kernel<R, 1>, map_blocks(n), 256, 0, s, n, w, y, live, st);
+    return e == cudaSuccess ? SINT_OK : cuda_fail(e, "Arnoldi step");
+  }
+  template int arnoldi_next<double>(long long, const double *, double *, const ArnoldiNext &, cudaStream_t,
+                                    const uint32_t *);
+  template int arnoldi_next<float>(long long, const float *, float *, const ArnoldiNext &, cudaStream_t,
+                                   const uint32_t *);
 
   template <typename S, typename D>
   __global__ void convert_kernel(long long n, const S *__restrict__ x, D *__restrict__ y)

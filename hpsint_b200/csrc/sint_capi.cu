@@ -50,19 +50,18 @@ namespace sint
     auto go = [&](auto nc) {
       constexpr int NC = decltype(nc)::value;
       const dim3    grid((unsigned)nb, (DIM == 2 && NC == 0) ? (unsigned)ncomp : 1u);
-      combine_kernel<DIM, R, NC><<<grid, 256, 0, s>>>(g, ncomp, partial, dst, tile_mask, sub, sc, fin ? 1 : 0);
+      return launch_dependent(combine_kernel<DIM, R, NC>, grid, 256, 0, s, g, ncomp, partial, dst, tile_mask, sub, sc,
+                              fin ? 1 : 0);
     };
     switch (ncomp)
       {
 #define SINT_NC(K)                                                                                                \
-  case K: go(std::integral_constant<int, K>{}); break;
+  case K: return go(std::integral_constant<int, K>{});
         SINT_NC(2) SINT_NC(3) SINT_NC(4) SINT_NC(5) SINT_NC(6) SINT_NC(7) SINT_NC(8) SINT_NC(9) SINT_NC(10)
         SINT_NC(11) SINT_NC(12) SINT_NC(13) SINT_NC(14) SINT_NC(15) SINT_NC(16)
 #undef SINT_NC
-        default: go(std::integral_constant<int, 0>{}); break;
+        default: return go(std::integral_constant<int, 0>{});
       }
-    count_launches(1);
-    return cudaGetLastError();
   }
 
   // dst = (dst - sub) * scale over the C blocks (the residual's epilogue hook
@@ -229,6 +228,7 @@ namespace sint
   __global__ void precond_apply_kernel(long long N, long long ld, int G, const R *__restrict__ inv,
                                        const R *__restrict__ r, R *__restrict__ z)
   {
+    dependent_start();
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N)
       return;
@@ -746,9 +746,8 @@ int sint_precond_apply_f64(sint_ctx *c, double *z, const double *r, sint_stream_
   else
     {
       const long long nb = (c->N + 255) / 256;
-      precond_apply_kernel<double><<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_inv64, r, z);
-      count_launches(1);
-      e = cudaGetLastError();
+      e = launch_dependent(precond_apply_kernel<double>, dim3((unsigned)nb), 256, 0, stream, c->N, c->ld, c->G,
+                           c->pc_inv64, r, z);
     }
   return e == cudaSuccess ? SINT_OK : cuda_fail(e, "sint_precond_apply_f64");
 }
@@ -772,9 +771,8 @@ int sint_precond_apply_f32(sint_ctx *c, float *z, const float *r, sint_stream_t 
   else
     {
       const long long nb = (c->N + 255) / 256;
-      precond_apply_kernel<float><<<dim3((unsigned)nb), 256, 0, stream>>>(c->N, c->ld, c->G, c->pc_inv32, r, z);
-      count_launches(1);
-      e = cudaGetLastError();
+      e = launch_dependent(precond_apply_kernel<float>, dim3((unsigned)nb), 256, 0, stream, c->N, c->ld, c->G,
+                           c->pc_inv32, r, z);
     }
   return e == cudaSuccess ? SINT_OK : cuda_fail(e, "sint_precond_apply_f32");
 }

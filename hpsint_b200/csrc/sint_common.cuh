@@ -799,6 +799,9 @@ namespace sint
                                                         const double *__restrict__ epi_sub = nullptr,
                                                         double epi_scale = 1.0, int epi = 0)
   {
+    // started as a programmatic dependent of the cell kernel (launch_dependent)
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     if constexpr (NC > 0)
       ncomp = NC;
     using T              = Tile<DIM>;

@@ -20,6 +20,7 @@
 #pragma once
 
 #include "sint_kernels.cuh"
+#include "sint_launch.h"
 
 namespace sint
 {
@@ -74,6 +75,7 @@ namespace sint
     constexpr int  C = L::C, P = L::P, TX = L::TX, TY = L::TY;
     constexpr bool JVP = L::JVP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    dependent_start();
     R *box = reinterpret_cast<R *>(smem_raw); // [field][node]
     R *up  = box + L::NF * L::BOX;            // [row][cell]: sums of the cell's upper nodes
 

@@ -126,10 +126,20 @@ namespace sint
   // w -= sum_i coef[i] * (V + i * stride), coef on the device
   template <typename R>
   int multiaxpy(long long n, R *w, const R *V, long long stride, int m, const double *coef, cudaStream_t s);
+  // Bookkeeping of an Arnoldi step after its first Gram-Schmidt pass (H null: none)
+  struct ArnoldiCheck
+  {
+    int           j = 0, ldh = 0;
+    const double *d_s     = nullptr; // the pass's dot products
+    double       *H       = nullptr; // Hessenberg matrix, column j at j * ldh
+    double        thresh2 = 0.0;
+    int          *reorth  = nullptr;
+  };
   // w -= sum_i coef[i] * V_i and norm2_out[0] = |w|^2 after the update (device scalar)
   template <typename R>
   int multiaxpy_norm2(Ctx *c, long long n, R *w, const R *V, long long stride, int m, const double *coef,
-                      double *norm2_out, cudaStream_t s, const uint32_t *live = nullptr);
+                      double *norm2_out, cudaStream_t s, const uint32_t *live = nullptr,
+                      const ArnoldiCheck &chk = ArnoldiCheck());
   // the same two, skipped on the device when *cond == 0 (launched unconditionally, decided on the GPU)
   template <typename R>
   int multidot_if(Ctx *c, long long n, const R *w, const R *V, long long stride, int m, double *out, const int *cond,
@@ -137,10 +147,20 @@ namespace sint
   template <typename R>
   int multiaxpy_norm2_if(Ctx *c, long long n, R *w, const R *V, long long stride, int m, const double *coef,
                          double *norm2_out, const int *cond, cudaStream_t s, const uint32_t *live = nullptr);
-  // y = x / d_div[0] (divisor on the device)
+  // End of Arnoldi step j: y = w / |w| with |w|^2 = d_s[MAX_MULTIDOT], and the
+  // Hessenberg column, Givens rotations and residual estimate.
+  struct ArnoldiNext
+  {
+    int           j = 0, ldh = 0;
+    const double *d_s = nullptr; // dot products of the (second) pass and |w|^2
+    double       *H = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr;
+    const int    *reorth = nullptr;
+    const double *tol    = nullptr;
+    double2      *out    = nullptr; // device-accessible host memory
+  };
   template <typename R>
-  int scale_by_device(long long n, const R *x, const double *d_div, R *y, cudaStream_t s,
-                      const uint32_t *live = nullptr);
+  int arnoldi_next(long long n, const R *w, R *y, const ArnoldiNext &st, cudaStream_t s,
+                   const uint32_t *live = nullptr);
   // y = a * x + b * y  (a, b on the host)
   template <typename R>
   int axpby(long long n, double a, const R *x, double b, R *y, cudaStream_t s, const uint32_t *live = nullptr);

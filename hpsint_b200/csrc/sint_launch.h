@@ -108,4 +108,34 @@ namespace sint
 
   // Counts kernel launches issued by this library.
   void count_launches(int n);
+
+  // Launch as a programmatic dependent of the stream's previous kernel: the
+  // grid is set up while that kernel ends.  The kernel must call
+  // cudaGridDependencySynchronize() before it touches memory (it then sees
+  // everything earlier in the stream, as after an ordinary launch).
+  template <typename... Params, typename... Args>
+  inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                      Args &&...args)
+  {
+    cudaLaunchConfig_t  cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim                                     = grid;
+    cfg.blockDim                                    = block;
+    cfg.dynamicSmemBytes                            = smem;
+    cfg.stream                                      = s;
+    cfg.attrs                                       = &attr;
+    cfg.numAttrs                                    = 1;
+    count_launches(1);
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+  }
+
+  // First statement of a kernel that launch_dependent starts: lets the next
+  // dependent launch set up, then waits for the stream's previous kernel.
+  __device__ __forceinline__ void dependent_start()
+  {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+  }
 } // namespace sint

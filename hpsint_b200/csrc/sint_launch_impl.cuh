@@ -143,9 +143,7 @@ namespace sint
       return e;
     args.blocks_x          = (g.nn[0] + L::TX - 2) / (L::TX - 1);
     const long long blocks = (long long)args.blocks_x * ((g.nn[1] + L::TY - 2) / (L::TY - 1));
-    k<<<dim3((unsigned)blocks), L::THREADS, smem, s>>>(g, p, args);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent(k, dim3((unsigned)blocks), L::THREADS, smem, s, g, p, args);
   }
 
   template <int DIM, int G, bool TENS, bool CUT, bool ADV>

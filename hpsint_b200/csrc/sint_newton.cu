@@ -37,7 +37,7 @@ namespace sint
     // Givens rotations, rotated right-hand side g, scalars {|w|, tol}, the re-orthogonalisation flag
     double  *d_H = nullptr, *d_cs = nullptr, *d_sn = nullptr, *d_g = nullptr, *d_sc = nullptr;
     int     *d_flag = nullptr;
-    double2 *d_out = nullptr, *h_out = nullptr; // per iteration {|g_{j+1}|, status}
+    double2 *h_out = nullptr; // per iteration {|g_{j+1}|, status}, pinned host memory the GPU writes
     double  *h_H   = nullptr;                   // pinned host copy of H and g at the end of a cycle
     cudaEvent_t ev[MAX_MULTIDOT] = {};
     // The Krylov loop runs on a private non-blocking stream (joined to the
@@ -86,7 +86,6 @@ namespace sint
     cudaFree(w->d_g);
     cudaFree(w->d_sc);
     cudaFree(w->d_flag);
-    cudaFree(w->d_out);
     cudaFreeHost(w->h_out);
     cudaFreeHost(w->h_H);
     for (cudaEvent_t &e : w->ev)
@@ -133,7 +132,6 @@ namespace sint
         (e = cudaMalloc(&w->d_g, sizeof(double) * (restart + 2))) != cudaSuccess ||
         (e = cudaMalloc(&w->d_sc, sizeof(double) * 4)) != cudaSuccess ||
         (e = cudaMalloc(&w->d_flag, sizeof(int) * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&w->d_out, sizeof(double2) * (restart + 1))) != cudaSuccess ||
         (e = cudaMallocHost(&w->h_out, sizeof(double2) * (restart + 1))) != cudaSuccess ||
         (e = cudaMallocHost(&w->h_H, sizeof(double) * ((restart + 1) * (restart + 1) + restart + 2))) != cudaSuccess)
       {
@@ -204,9 +202,11 @@ namespace sint
   }
 
   // --- device-resident Arnoldi bookkeeping ------------------------------------
-  // One thread does the O(restart) scalar work of an Arnoldi step on the GPU,
-  // so the host never waits for a Hessenberg column: it only reads the
-  // residual estimate of iteration j while iteration j + 1 already runs.
+  // The O(restart) scalar work of an Arnoldi step runs on the GPU, inside the
+  // kernels that update the vectors (ArnoldiCheck, ArnoldiNext), so the host
+  // never waits for a Hessenberg column: it only reads the residual estimate
+  // of iteration j, which the GPU writes to host memory, while iteration j + 1
+  // already runs.
 
   // start of a cycle: g = (beta, 0, ...), sc[1] = tol (first cycle) and status
   __global__ void gmres_cycle_init_kernel(int m, double beta, double *g)
@@ -215,80 +215,15 @@ namespace sint
       g[i] = i == 0 ? beta : 0.0;
   }
 
-  // after the first Gram-Schmidt pass: Hessenberg column j = h and deal.II's
-  // re-orthogonalisation test (Kelley 1995, as in SolverGMRES): once |w| after
-  // the pass falls below 10 sqrt(eps) of |w| before it, every later iteration
-  // of this solve takes a second pass (the flag is sticky).  thresh2 =
-  // 100 eps of the Krylov vectors' precision; |w|^2 before = |h|^2 + |w'|^2.
-  __global__ void arnoldi_check_kernel(int j, int ldh, const double *__restrict__ d_s, double *__restrict__ H,
-                                       double thresh2, int *__restrict__ reorth)
-  {
-    if (threadIdx.x != 0)
-      return;
-    double *hcol = H + (long long)j * ldh;
-    double  hh   = 0.0;
-    for (int i = 0; i <= j; ++i)
-      {
-        hcol[i] = d_s[i];
-        hh += d_s[i] * d_s[i];
-      }
-    const double nw2 = d_s[MAX_MULTIDOT];
-    if (nw2 < thresh2 * (hh + nw2))
-      *reorth = 1;
-  }
-
-  // after the (optional) second pass: |w|, Givens rotations, residual estimate.
-  // out[j] = {|g_{j+1}|, status}: 0 continue, 1 converged, 2 breakdown, 3 non-finite
-  __global__ void arnoldi_finish_kernel(int j, int ldh, const double *__restrict__ d_s, double *__restrict__ H,
-                                        double *__restrict__ cs, double *__restrict__ sn, double *__restrict__ g,
-                                        const int *__restrict__ reorth, double *__restrict__ sc,
-                                        double2 *__restrict__ out)
-  {
-    if (threadIdx.x != 0)
-      return;
-    double *hcol = H + (long long)j * ldh;
-    if (*reorth)
-      for (int i = 0; i <= j; ++i)
-        hcol[i] += d_s[i];
-    const double nw = sqrt(fmax(d_s[MAX_MULTIDOT], 0.0));
-    hcol[j + 1]     = nw;
-    for (int i = 0; i < j; ++i)
-      {
-        const double a = hcol[i], b = hcol[i + 1];
-        hcol[i]         = cs[i] * a + sn[i] * b;
-        hcol[i + 1]     = -sn[i] * a + cs[i] * b;
-      }
-    const double a = hcol[j], b = hcol[j + 1];
-    const double rr = hypot(a, b);
-    cs[j]           = rr == 0.0 ? 1.0 : a / rr;
-    sn[j]           = rr == 0.0 ? 0.0 : b / rr;
-    hcol[j]         = rr;
-    hcol[j + 1]     = 0.0;
-    g[j + 1]        = -sn[j] * g[j];
-    g[j]            = cs[j] * g[j];
-    const double res = fabs(g[j + 1]);
-    double       status;
-    if (!isfinite(res) || !isfinite(nw))
-      status = 3.0;
-    else if (res <= sc[1])
-      status = 1.0;
-    else if (nw == 0.0)
-      status = 2.0;
-    else
-      status = 0.0;
-    sc[0]  = nw;
-    out[j] = make_double2(res, status);
-  }
-
   // Restarted, left-preconditioned GMRES for J x = b with x0 = 0; classical
   // Gram-Schmidt with deal.II's re-orthogonalisation test (second pass from
   // the first iteration whose norm drops below 10 sqrt(eps) of its starting
   // value on).  Returns SINT_OK / SINT_ERR_NO_CONVERGENCE; *its = iterations.
   //
   // Each Arnoldi iteration is a fixed sequence of kernels (J v, P^-1, fused
-  // multi-dot, fused multi-axpy + norm, check, conditional second pass,
-  // finish, normalisation of the next basis vector) plus a 16-byte copy of
-  // its residual estimate; the host enqueues iteration j + 1 before it waits
+  // multi-dot, fused multi-axpy + norm + check, conditional second pass,
+  // normalisation of the next basis vector + bookkeeping), launched as
+  // programmatic dependents; the host enqueues iteration j + 1 before it waits
   // for iteration j's estimate, unless the residual history predicts that j
   // converges.  An iteration enqueued past convergence only writes basis
   // vector j + 2 and Hessenberg column j + 1, which the solution update
@@ -334,21 +269,16 @@ namespace sint
       if ((right ? ((r = prec<R>(c, t, vj, s)) || (r = jvp<R>(c, w, t, s)))
                  : ((r = jvp<R>(c, t, vj, s)) || (r = prec<R>(c, w, t, s)))) ||
           (r = multidot<R>(c, n, w, V, n, j + 1, ws->d_s, s, live)) ||
-          (r = multiaxpy_norm2<R>(c, n, w, V, n, j + 1, ws->d_s, ws->d_s + MAX_MULTIDOT, s, live)))
+          (r = multiaxpy_norm2<R>(c, n, w, V, n, j + 1, ws->d_s, ws->d_s + MAX_MULTIDOT, s, live,
+                                  ArnoldiCheck{j, ldh, ws->d_s, ws->d_H, reorth_thresh2, ws->d_flag})))
         return r;
-      arnoldi_check_kernel<<<1, 32, 0, s>>>(j, ldh, ws->d_s, ws->d_H, reorth_thresh2, ws->d_flag);
-      count_launches(1);
       if ((r = multidot_if<R>(c, n, w, V, n, j + 1, ws->d_s, ws->d_flag, s, live)) ||
           (r = multiaxpy_norm2_if<R>(c, n, w, V, n, j + 1, ws->d_s, ws->d_s + MAX_MULTIDOT, ws->d_flag, s, live)))
         return r;
-      arnoldi_finish_kernel<<<1, 32, 0, s>>>(j, ldh, ws->d_s, ws->d_H, ws->d_cs, ws->d_sn, ws->d_g, ws->d_flag,
-                                             ws->d_sc, ws->d_out);
-      count_launches(1);
-      if ((r = scale_by_device<R>(n, w, ws->d_sc, V + (long long)(j + 1) * n, s, live)))
-        return r;
-      const cudaError_t e =
-        cudaMemcpyAsync(ws->h_out + j, ws->d_out + j, sizeof(double2), cudaMemcpyDeviceToHost, s);
-      return e == cudaSuccess ? SINT_OK : cuda_fail(e, "GMRES: enqueue");
+      return arnoldi_next<R>(n, w, V + (long long)(j + 1) * n,
+                             ArnoldiNext{j, ldh, ws->d_s, ws->d_H, ws->d_cs, ws->d_sn, ws->d_g, ws->d_flag,
+                                         ws->d_sc + 1, ws->h_out},
+                             s, live);
     };
 
     // Iteration j: replay its graph (capture or update it first when needed),
