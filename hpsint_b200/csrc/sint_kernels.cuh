@@ -211,11 +211,11 @@ namespace sint
     for (int i = 0; i < G; ++i)
       s2 += eta[i] * eta[i];
     const R omc = R(1) - c;
-    const R fcc = R(2) * p.A * (c * c) + R(4) * p.A * c * (R(2) * c - R(2)) + R(2) * p.A * (omc * omc) + R(2) * p.B;
+    // f_cc = 2 A c^2 + 4 A c (2 c - 2) + 2 A (1 - c)^2 + 2 B = 2 (A + B) - 12 A c (1 - c)
+    const R fcc = R(2) * (p.A + p.B) - (R(12) * p.A) * c * omc;
     const R B12 = p.B * R(12);
     // f_{c eta_i} = 12 B eta_i (eta_i - 1) (free_energy.h:150-152), shared by the mu
-    // and eta rows; f_{eta_i eta_i} = B (12 - 12 c + 2 eta_i (12 c - 24) + 24 eta_i^2
-    // + 12 sum eta^2) (:154-158) in Horner form: f0 + eta_i (f1 + f2 eta_i)
+    // and eta rows
     R fce[gdim(G)];
 #pragma unroll
     for (int i = 0; i < G; ++i)
@@ -223,7 +223,6 @@ namespace sint
         const R be = B12 * eta[i];
         fce[i]     = be * eta[i] - be;
       }
-    const R fee0 = B12 * ((R(1) - c) + s2), fee1 = p.B * (R(24) * c - R(48)), fee2 = p.B * R(24);
 
     // 1) c row (generic.h:120-134)
     {
@@ -248,15 +247,18 @@ namespace sint
 #pragma unroll
       for (int i = 0; i < G; ++i)
         S += eta[i] * deta[i];
-      const R cL24B = p.L * R(24) * p.B;
+      // w0 deta_i + L (f_{c eta_i} dc + f_{eta_i eta_i} deta_i) + 24 B L eta_i (S -
+      // eta_i deta_i) with f_{eta_i eta_i} = B (12 - 12 c + 2 eta_i (12 c - 24) + 24
+      // eta_i^2 + 12 sum eta^2) (free_energy.h:154-158): the 24 B L eta_i^2 deta_i
+      // of the last two cancel
+      const R al0 = p.w0 + p.L * (B12 * (omc + s2)), al1 = (p.L * p.B) * (R(24) * c - R(48));
+      const R Ldc = p.L * dc, gS = (p.L * R(24) * p.B) * S;
 #pragma unroll
       for (int i = 0; i < G; ++i)
         {
-          const R e   = eta[i];
-          const R fee = fee0 + e * (fee1 + fee2 * e);
-          R       v   = deta[i] * p.w0 + p.L * (fce[i] * dc + fee * deta[i]);
-          if constexpr (G > 1)
-            v += (cL24B * e) * (S - e * deta[i]);
+          const R al = al0 + eta[i] * al1;
+          R       v  = deta[i] * al + fce[i] * Ldc;
+          v += gS * eta[i];
           emit(DIM + 2 + i, v);
         }
     }
@@ -307,10 +309,12 @@ namespace sint
 #pragma unroll
     for (int i = 0; i < G; ++i)
       {
-        s2 += eta[i] * eta[i];
-        s3 += eta[i] * eta[i] * eta[i];
+        const R e2 = eta[i] * eta[i];
+        s2 += e2;
+        s3 += e2 * eta[i];
       }
     const R omc = R(1) - c;
+    const R LB12 = p.L * (p.B * R(12)), os = omc + s2;
     // 1) c row (generic.h:275-285)
     {
       const R v = time(-1, R(0));
@@ -323,8 +327,8 @@ namespace sint
     }
     // 2) mu row value (generic.h:288, free_energy.h:124-134)
     {
-      const R df_dc = p.A * (c * c) * (R(2) * c - R(2)) + R(2) * p.A * c * (omc * omc) +
-                      p.B * (R(2) * c - R(6) * s2 + R(4) * s3);
+      // A c^2 (2 c - 2) + 2 A c (1 - c)^2 = 2 A c (1 - c) (1 - 2 c)
+      const R df_dc = (R(2) * p.A) * c * omc * (R(1) - R(2) * c) + p.B * (R(2) * c - R(6) * s2 + R(4) * s3);
       emit(DIM + 1, p.walg * mu - df_dc);
     }
     // 3) eta row values (generic.h:293-302, free_energy.h:136-141)
@@ -332,7 +336,7 @@ namespace sint
     for (int i = 0; i < G; ++i)
       {
         const R e = eta[i];
-        emit(DIM + 2 + i, time(i, p.L * (e * (p.B * R(12)) * (e * (c - R(2)) + omc + s2))));
+        emit(DIM + 2 + i, time(i, (LB12 * e) * (e * (c - R(2)) + os)));
       }
   }
 
@@ -497,23 +501,24 @@ namespace sint
     for (int i = 0; i < G; ++i)
       {
         const R e = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
-        s2 += e * e;
-        s3 += e * e * e;
+        const R e2 = e * e;
+        s2 += e2;
+        s3 += e2 * e;
       }
     const R omc = R(1) - c;
+    const R LB12 = p.L * (p.B * R(12)), os = omc + s2;
 #pragma unroll 3
     for (int i = 0; i < G; ++i)
       {
         const R e = fval<DIM>(F, FM::base(FM::lin_eta(i)), q, cell);
-        R       v = p.L * (e * (p.B * R(12)) * (e * (c - R(2)) + omc + s2));
+        R       v = (LB12 * e) * (e * (c - R(2)) + os);
         if constexpr (WTD >= 1)
           v += e * p.w0;
         if constexpr (WTD == 2)
           v += fval<DIM>(F, FM::base(FM::h_eta(i)), q, cell);
         pstore<DIM>(F, FM::result(DIM + 2 + i), q, cell, v);
       }
-    const R df_dc = p.A * (c * c) * (R(2) * c - R(2)) + R(2) * p.A * c * (omc * omc) +
-                    p.B * (R(2) * c - R(6) * s2 + R(4) * s3);
+    const R df_dc = (R(2) * p.A) * c * omc * (R(1) - R(2) * c) + p.B * (R(2) * c - R(6) * s2 + R(4) * s3);
     pstore<DIM>(F, FM::result(0), q, cell, v0);
 #pragma unroll
     for (int d = 0; d < DIM; ++d)

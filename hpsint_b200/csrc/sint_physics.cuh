@@ -33,22 +33,17 @@ namespace sint
     return s;
   }
 
-  // Reciprocal and inverse square root of a positive number by Newton-Raphson
-  // refinement of the single-precision hardware seed (rcp.approx /
-  // rsqrt.approx, relative error ~2^-23 including the rounding of the
-  // argument to float):
-  //   reciprocal:          y <- y + y (1 - x y)
-  //   inverse square root: y <- y + (y / 2) (1 - x y^2)
-  // One step squares the relative error: ~3e-14 in double (far inside the
-  // operator's 1e-12 parity bound), float rounding level in float.  The seeds
-  // need the argument and the result inside the normal float range, [2^-126,
-  // 2^126] for the reciprocal and [2^-126, 2^128) for the inverse square root.
-  // In double the argument is scaled by 2^-56 before seeding and the result
-  // back by the exact power of two, which moves that range to [2^-70, 2^182]
-  // (8.5e-22 .. 6e54): the callers filter squared norms below 1e-20, and a
-  // squared gradient norm above 6e54 would need a gradient steeper than
-  // 2e27 per unit length.  (No branch: a guarded exact division here cost 8 %
-  // of the FP64 Jacobian product.)
+  // Reciprocal and inverse square root of a positive number: a hardware seed
+  // and one step of a power series in its error e,
+  //   reciprocal:          e = 1 - x y,    y <- y (1 + e + e^2 (FP64))
+  //   inverse square root: e = 1 - x y^2,  y <- y (1 + e / 2 + 3 e^2 / 8 (FP64))
+  // FP32: rcp.approx / rsqrt.approx (error ~2^-23) and the linear step, float
+  // rounding level.  FP64: rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64, which
+  // take and give doubles of full exponent range with ~20 good bits, and the
+  // quadratic step: error below 2^-52 + e^3.  Against the float seeds with a
+  // linear step and their scaling by 2^56, which these replace, that saves
+  // two conversions and one operation per reciprocal and is more exact (3e-14
+  // before).
   __device__ __forceinline__ float rcp_seed(float x)
   {
     float y;
@@ -88,9 +83,10 @@ namespace sint
   {
     if constexpr (std::is_same_v<R, double>)
       {
-        const double xs = x * 0x1p-56;
-        const double s  = double(rcp_seed(float(xs)));
-        return (s + s * (1.0 - xs * s)) * 0x1p-56;
+        double y;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double e = fma(-x, y, 1.0);
+        return fma(y, fma(e, e, e), y);
       }
     else
       {
@@ -104,9 +100,10 @@ namespace sint
   {
     if constexpr (std::is_same_v<R, double>)
       {
-        const double xs = x * 0x1p-56;
-        const double s  = double(rsqrt_seed(float(xs)));
-        return (s + (0.5 * s) * (1.0 - (xs * s) * s)) * 0x1p-28;
+        double y;
+        asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+        const double e = fma(-(x * y), y, 1.0);
+        return fma(y * e, fma(0.375, e, 0.5), y);
       }
     else
       {
@@ -159,7 +156,7 @@ namespace sint
   template <typename R>
   __device__ __forceinline__ R phi_clamped(R c)
   {
-    return clamp01(c * c * c * (R(10) - R(15) * c + R(6) * c * c));
+    return clamp01(c * c * c * (R(10) + c * (R(6) * c - R(15))));
   }
 
   // ---------------------------------------------------------------------
@@ -241,6 +238,9 @@ namespace sint
   {
     const R phi = phi_clamped(c);
     const R omc = R(1) - c;
+    const R cq  = c * omc; // c (1 - c)
+    // Mvol phi + Mvap (1 - phi)
+    const R fvv = p.Mvap + (p.Mvol - p.Mvap) * phi;
     if constexpr (!TENS)
       {
         // sum_{i>j} eta_i eta_j = sum_i eta_i (eta_0 + .. + eta_{i-1})
@@ -251,9 +251,9 @@ namespace sint
             eta_ij += eta[i] * eta_sum;
             eta_sum += eta[i];
           }
-        const R M = p.Mvol * phi + p.Mvap * (R(1) - phi) + p.Msurf * R(4) * c * c * omc * omc + (R(2) * p.Mgb) * eta_ij;
-        const R dphidc = R(30) * c * c * omc * omc;
-        const R dMdc   = p.Mvol * dphidc - p.Mvap * dphidc + p.Msurf * R(8) * c * (R(1) - R(3) * c + R(2) * c * c);
+        const R c2   = cq * cq;
+        const R M    = fvv + (p.Msurf * R(4)) * c2 + (R(2) * p.Mgb) * eta_ij;
+        const R dMdc = ((p.Mvol - p.Mvap) * R(30)) * c2 + (p.Msurf * R(8)) * cq * (R(1) - R(2) * c);
         R       factor = R(0);
 #pragma unroll
         for (int i = 0; i < G; ++i)
@@ -267,15 +267,14 @@ namespace sint
       {
         R nc[DIM], n2, rs;
         unit_vector<DIM>(gc, nc, n2, rs);
-        const R c2 = R(4) * c * c * omc * omc; // 4 c^2 (1-c)^2
+        const R c2 = (R(4) * cq) * cq; // 4 c^2 (1-c)^2
         // 1) M
-        const R fvv   = p.Mvol * phi + p.Mvap * (R(1) - phi);
         const R fsurf = p.Msurf * c2;
         const R nc_gdmu = dotv<DIM>(nc, gdmu);
         const R nc_gmu  = dotv<DIM>(nc, gmu);
         // 2) dM/dc (hpsint uses dphidc = 30 * 4 c^2 (1-c)^2 here, mobility.h:852-854)
-        const R fvv2  = (p.Mvol - p.Mvap) * (R(30) * c2);
-        R       dfs   = p.Msurf * R(8) * c * omc * (R(1) - R(2) * c);
+        const R fvv2  = ((p.Mvol - p.Mvap) * R(30)) * c2;
+        R       dfs   = (p.Msurf * R(8)) * cq * (R(1) - R(2) * c);
         dfs           = sel(fsurf < R(1e-6), R(0), dfs);
         // 3) dM/dgrad c; |grad c| < 1e-4 (|grad c|^2 < 1e-8) counts as 1
         const R fs3   = sel(fsurf < R(1e-6), R(0), fsurf);
