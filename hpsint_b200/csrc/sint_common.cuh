@@ -784,29 +784,29 @@ namespace sint
 
   // Second pass of the scatter: nodes on an interior tile face sum the
   // partials of the 2, 4 or 8 tiles that share them, in a fixed order.  One
-  // thread per (node, component): blockIdx.y is the component, so the
-  // partial loads of different components are independent.
-  // tile_mask (grain cut-off): a tile's partial of grain component 2 + b
-  // exists only when bit b of tile_mask[tile] is set; nullptr = all exist.
+  // thread per node and group of CH components (blockIdx.y): all partial loads
+  // of a thread are in flight together.  Bound by latency: a thread with all
+  // components of a node holds too few loads at once (47 registers), one per
+  // component repeats the node's classification too often.
+  // MASKED (grain cut-off): a tile's partial of grain component 2 + b exists
+  // only when bit b of tile_mask[tile] is set.  Most shared nodes of a packing
+  // lie between tiles without a relevant grain, so there one thread serves all
+  // components: c and mu together, then a grain only where a sharing tile wrote
+  // it (256^3 cells, 12 components: 0.77 ms in
+  // groups of six components).
   // epi (the residual's epilogue hook, nullptr for none): the combined sums
   // are stored as (sum - sub) * scale.
-  // NC > 0: the component count at compile time, one thread per node, so a
-  // thread's partial loads of all components can be in flight together (same
-  // sums, same order).
-  template <int DIM, typename R, int NC = 0>
+  template <int DIM, typename R, int CH, bool MASKED>
   __global__ void __launch_bounds__(256) combine_kernel(const Grid g, int ncomp, const R *__restrict__ partial,
                                                         R *__restrict__ dst, const uint16_t *__restrict__ tile_mask,
-                                                        const double *__restrict__ epi_sub = nullptr,
-                                                        double epi_scale = 1.0, int epi = 0)
+                                                        const double *__restrict__ epi_sub, double epi_scale, int epi)
   {
     // started as a programmatic dependent of the cell kernel (launch_dependent)
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
-    if constexpr (NC > 0)
-      ncomp = NC;
-    using T              = Tile<DIM>;
-    const long long idx  = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int       comp = blockIdx.y;
+    using T             = Tile<DIM>;
+    constexpr int   NT  = 1 << DIM; // candidate tiles of a node
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= g.N)
       return;
     int c[3];
@@ -826,74 +826,80 @@ namespace sint
         c[2] = int(idx / ((long long)g.nn[0] * g.nn[1]));
       }
     const int TT[3]  = {T::TX, T::TY, T::TZ};
-    int       nt[3]  = {1, 1, 1}; // number of candidate tiles per direction
-    int       t0[3]  = {0, 0, 0}; // first candidate tile
-    int       lo[3]  = {0, 0, 0}; // local box coordinate in the first candidate
-    bool      shared = false;
+    bool      two[3] = {false, false, false}; // two candidate tiles in the direction
+    int       t0[3]  = {0, 0, 0};             // first candidate tile
+    int       lo[3]  = {0, 0, 0};             // local box coordinate in the first candidate
 #pragma unroll
     for (int d = 0; d < DIM; ++d)
       {
-        if (c[d] % TT[d] == 0 && c[d] > 0 && c[d] < g.n[d])
-          {
-            shared = true;
-            nt[d]  = 2;
-            t0[d]  = c[d] / TT[d] - 1;
-            lo[d]  = TT[d];
-          }
-        else
-          {
-            t0[d] = min(c[d] / TT[d], g.nt[d] - 1);
-            lo[d] = c[d] - t0[d] * TT[d];
-          }
+        two[d] = c[d] % TT[d] == 0 && c[d] > 0 && c[d] < g.n[d];
+        t0[d]  = two[d] ? c[d] / TT[d] - 1 : min(c[d] / TT[d], g.nt[d] - 1);
+        lo[d]  = c[d] - t0[d] * TT[d];
       }
-    if (!shared)
+    if (!(two[0] || two[1] || two[2]))
       return;
-    // the (up to 8) tiles sharing the node, in a fixed order: the node's slot
-    // in each tile's partials and the grains each tile wrote
-    long long slot[8];
-    unsigned  tm[8];
-    bool      has[8];
+    // the node's slot in the first candidate's partials and the steps to the
+    // next candidate per direction
+    const long long tile0 = t0[0] + (long long)g.nt[0] * (t0[1] + (long long)g.nt[1] * t0[2]);
+    const long long dt[3] = {1, g.nt[0], (long long)g.nt[0] * g.nt[1]};
+    const long long per   = (long long)ncomp * T::BOX;
+    const long long slot0 = tile0 * per + lo[0] + T::BX * (lo[1] + T::BY * lo[2]);
+    const long long ds[3] = {per - T::TX, dt[1] * per - T::BX * T::TY, dt[2] * per - T::BX * T::BY * T::TZ};
+    const int       cp0   = MASKED ? 0 : blockIdx.y * CH;
+    auto            store = [&](int cp, R sum) {
+      const long long at = cp * g.ld + idx;
+      if (epi)
+        sum = (sum - (epi_sub ? R(epi_sub[at]) : R(0))) * R(epi_scale);
+      dst[at] = sum;
+    };
+    long long off[NT];
+    unsigned  wrote[NT], any = 0u; // bits of the components the candidates wrote (c and mu always)
+    R         v[NT][CH];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int bb = 0; bb < 2; ++bb)
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc)
-          {
-            const int k = 4 * a + 2 * bb + cc;
-            has[k]      = a < nt[2] && bb < nt[1] && cc < nt[0];
-            const int       ti = t0[0] + cc, tj = t0[1] + bb, tk = t0[2] + a;
-            const int       bx = lo[0] - cc * TT[0], by = lo[1] - bb * TT[1], bz = lo[2] - a * TT[2];
-            const long long tile = ti + (long long)g.nt[0] * (tj + (long long)g.nt[1] * tk);
-            slot[k] = tile * ncomp * (long long)T::BOX + bx + T::BX * (by + T::BY * bz);
-            tm[k]   = (has[k] && tile_mask) ? unsigned(tile_mask[tile]) : ~0u;
-          }
-    // grains written by any of the sharing tiles: the others sum to zero
-    // without a look at the candidates (most shared nodes of a packing lie
-    // between tiles without a relevant grain)
-    unsigned any = 0u;
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (has[k])
-        any |= tm[k];
-    // NC > 0: one thread loops over all components (known at compile time);
-    // otherwise in 2D one component per thread (blockIdx.y), in 3D the loop
-    constexpr bool PER_COMP = DIM == 2 && NC == 0;
-    const int      c_end    = PER_COMP ? comp + 1 : ncomp;
-#pragma unroll
-    for (int cp = PER_COMP ? comp : 0; cp < (NC > 0 ? NC : c_end); ++cp)
+    for (int k = 0; k < NT; ++k)
       {
-        R sum = R(0);
-        if (cp < 2 || ((any >> (cp - 2)) & 1u) != 0u)
-          {
+        const bool has  = (!(k & 1) || two[0]) && (!(k & 2) || two[1]) && (!(k & 4) || two[2]);
+        long long  tile = tile0;
+        off[k]          = slot0;
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              if (has[k] && (cp < 2 || ((tm[k] >> (cp - 2)) & 1u) != 0u))
-                sum += partial[slot[k] + cp * (long long)T::BOX];
+        for (int d = 0; d < DIM; ++d)
+          if ((k >> d) & 1)
+            {
+              off[k] += ds[d];
+              tile += dt[d];
+            }
+        wrote[k] = !has ? 0u : (MASKED ? (unsigned(tile_mask[tile]) << 2) | 3u : ~0u);
+        any |= wrote[k];
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+          v[k][i] = has && (MASKED || cp0 + i < ncomp) ? partial[off[k] + (cp0 + i) * T::BOX] : R(0);
+      }
+#pragma unroll
+    for (int i = 0; i < CH; ++i)
+      if (MASKED || cp0 + i < ncomp)
+        {
+          R sum = R(0);
+#pragma unroll
+          for (int k = 0; k < NT; ++k)
+            sum += v[k][i];
+          store(cp0 + i, sum);
+        }
+    if constexpr (MASKED)
+      {
+        static_assert(CH == 2, "c and mu first");
+#pragma unroll 1
+        for (int cp = 2; cp < ncomp; ++cp)
+          {
+            R sum = R(0);
+            if ((any >> cp) & 1u)
+              {
+#pragma unroll
+                for (int k = 0; k < NT; ++k)
+                  if ((wrote[k] >> cp) & 1u)
+                    sum += partial[off[k] + cp * T::BOX];
+              }
+            store(cp, sum);
           }
-        if (epi)
-          sum = (sum - (epi_sub ? R(epi_sub[cp * g.ld + idx]) : R(0))) * R(epi_scale);
-        dst[cp * g.ld + idx] = sum;
       }
   }
 } // namespace sint
