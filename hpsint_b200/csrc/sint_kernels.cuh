@@ -4,6 +4,7 @@
 
 #include "sint_cellfact.cuh"
 #include "sint_common.cuh"
+#include "sint_launch.h"
 #include "sint_physics.cuh"
 
 namespace sint
@@ -919,6 +920,8 @@ namespace sint
     using FM = typename SM::FM;
     using PL = ThreePhasePlan<DIM, G, TENS, true, false, ADV, sizeof(R)>;
     constexpr int C = G + 2, NBUF = SM::BUFFERS;
+    if constexpr (CUT)
+      siblings_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *s_buf = reinterpret_cast<R *>(smem_raw); // NBUF x BOXES
     R *F     = s_buf + NBUF * SM::BOXES;
@@ -1055,6 +1058,8 @@ namespace sint
           tile = nidx;
       }
     cp_async_wait<0>();
+    if constexpr (CUT)
+      siblings_end();
   }
 
   // -------------------------------------------------------------------------
@@ -1091,6 +1096,8 @@ namespace sint
     using FM = typename SM::FM;
     static_assert(G <= 4 && SM::BUFFERS == 2, "pairs serve few grains");
     constexpr int C = G + 2;
+    if constexpr (CUT)
+      siblings_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     F2 *s_buf = reinterpret_cast<F2 *>(smem_raw); // 2 x BOXES pairs
     F2 *F     = s_buf + 2 * SM::BOXES;
@@ -1172,6 +1179,8 @@ namespace sint
           }
       }
     cp_async_wait<0>();
+    if constexpr (CUT)
+      siblings_end();
   }
 
   // -------------------------------------------------------------------------
@@ -1194,6 +1203,8 @@ namespace sint
     using FM = typename SM::FM;
     using PL = ThreePhasePlan<DIM, G, TENS, false, WTD == 2, ADV, sizeof(double)>;
     constexpr int C = G + 2;
+    if constexpr (CUT)
+      siblings_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R *s_u = reinterpret_cast<R *>(smem_raw);
     R *s_h = s_u + C * T::BOXS;
@@ -1275,6 +1286,8 @@ namespace sint
         // phase 3 before the barrier above; K (aliasing F) is next written in
         // phase 1, after the barrier that follows the staging
       }
+    if constexpr (CUT)
+      siblings_end();
   }
 
   // -------------------------------------------------------------------------

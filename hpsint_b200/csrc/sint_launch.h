@@ -113,9 +113,10 @@ namespace sint
   // grid is set up while that kernel ends.  The kernel must call
   // cudaGridDependencySynchronize() before it touches memory (it then sees
   // everything earlier in the stream, as after an ordinary launch).
+  // dependent = false: an ordinary launch.
   template <typename... Params, typename... Args>
-  inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                                      Args &&...args)
+  inline cudaError_t launch_dependent_if(bool dependent, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                         cudaStream_t s, Args &&...args)
   {
     cudaLaunchConfig_t  cfg{};
     cudaLaunchAttribute attr{};
@@ -126,9 +127,28 @@ namespace sint
     cfg.dynamicSmemBytes                            = smem;
     cfg.stream                                      = s;
     cfg.attrs                                       = &attr;
-    cfg.numAttrs                                    = 1;
+    cfg.numAttrs                                    = dependent ? 1 : 0;
     count_launches(1);
     return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+  }
+  template <typename... Params, typename... Args>
+  inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                      Args &&...args)
+  {
+    return launch_dependent_if(true, kernel, grid, block, smem, s, args...);
+  }
+
+  // The grain cut-off's class kernels of one operator call write disjoint
+  // outputs, so each may run beside the one launched before it: the first is
+  // an ordinary launch (all inputs are complete when it starts), every other a
+  // dependent one that waits for nothing at its start (siblings_begin) but
+  // does not complete before its predecessor: its block 0 waits at the end
+  // (siblings_end), so what follows the last kernel follows them all.
+  __device__ __forceinline__ void siblings_begin() { cudaTriggerProgrammaticLaunchCompletion(); }
+  __device__ __forceinline__ void siblings_end()
+  {
+    if (blockIdx.x == 0)
+      cudaGridDependencySynchronize();
   }
 
   // First statement of a kernel that launch_dependent starts: lets the next

@@ -50,9 +50,10 @@ namespace sint
     });
   }
 
+  // sibling: a class kernel of the cut-off that may run beside the one before it
   template <int DIM, int G, bool TENS, typename R, bool CUT, bool ADV>
   cudaError_t launch_jvp_g(const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
-                           const CutTiles &ct, const AdvData &adv, cudaStream_t s)
+                           const CutTiles &ct, const AdvData &adv, cudaStream_t s, bool sibling = false)
   {
     const size_t smem = ThreePhaseSmem<DIM, G, TENS, true, false, ADV, sizeof(R)>::TOTAL * sizeof(R);
     auto         k    = jvp_kernel<DIM, G, TENS, R, CUT, ADV>;
@@ -62,14 +63,13 @@ namespace sint
           persistent_grid(cache, k, smem, jvp_blocks_per_sm<DIM, G, TENS, R, ADV>(), Tile<DIM>::THREADS, grid_cap))
       return e;
     const long long blocks = g.n_tiles < grid_cap ? g.n_tiles : grid_cap;
-    k<<<dim3((unsigned)blocks), Tile<DIM>::THREADS, smem, s>>>(g, p, lin, src, dst, partial, ct, adv);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent_if(sibling, k, dim3((unsigned)blocks), Tile<DIM>::THREADS, smem, s, g, p, lin, src, dst,
+                               partial, ct, adv);
   }
 
   template <int DIM, int G, bool TENS, bool CUT = false>
   cudaError_t launch_jvp_pair_g(const Grid &g, const Phys &p, const float *lin, const float *src, float *dst,
-                                float *partial, cudaStream_t s, const CutTiles &ct = CutTiles())
+                                float *partial, cudaStream_t s, const CutTiles &ct = CutTiles(), bool sibling = false)
   {
     const size_t smem = ThreePhaseSmem<DIM, G, TENS, true, false, false, sizeof(F2)>::TOTAL * sizeof(F2);
     auto         k    = jvp_pair_kernel<DIM, G, TENS, CUT>;
@@ -81,15 +81,14 @@ namespace sint
     // the class size of the cut-off lives on the device: a full persistent grid
     const long long pairs  = CUT ? (long long)grid_cap : (g.n_tiles + 1) / 2;
     const long long blocks = pairs < grid_cap ? pairs : grid_cap;
-    k<<<dim3((unsigned)blocks), Tile<DIM>::THREADS, smem, s>>>(g, p, lin, src, dst, partial, ct);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent_if(sibling, k, dim3((unsigned)blocks), Tile<DIM>::THREADS, smem, s, g, p, lin, src, dst,
+                               partial, ct);
   }
 
   template <int DIM, int G, bool TENS, int WTD, bool CUT, bool ADV>
   cudaError_t launch_residual_g(const Grid &g, const Phys &p, const double *src, const double *const *hist,
                                 double *dst, double *partial, const CutTiles &ct, const AdvData &adv,
-                                cudaStream_t s)
+                                cudaStream_t s, bool sibling = false)
   {
     const size_t  smem     = ThreePhaseSmem<DIM, G, TENS, false, WTD == 2, ADV, sizeof(double)>::TOTAL * sizeof(double);
     auto          k        = residual_kernel<DIM, G, TENS, WTD, CUT, ADV>;
@@ -102,16 +101,16 @@ namespace sint
     const double *h1     = (WTD == 2 && p.order > 1) ? hist[1] : nullptr;
     const double *h2     = (WTD == 2 && p.order > 2) ? hist[2] : nullptr;
     const long long blocks = g.n_tiles < grid_cap ? g.n_tiles : grid_cap;
-    k<<<dim3((unsigned)blocks), Tile<DIM>::THREADS, smem, s>>>(g, p, src, h0, h1, h2, dst, partial, ct, adv);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent_if(sibling, k, dim3((unsigned)blocks), Tile<DIM>::THREADS, smem, s, g, p, src, h0, h1, h2, dst,
+                               partial, ct, adv);
   }
 
   // The 3D class of the grain cut-off without a relevant grain (MODE: -1 = J v,
   // 0..2 = residual); the class size lives on the device, so the grid is the
   // persistent one.
   template <bool TENS, typename R, int MODE>
-  cudaError_t launch_light(const Grid &g, const Phys &p, const LightArgs<R> &args, const CutTiles &ct, cudaStream_t s)
+  cudaError_t launch_light(const Grid &g, const Phys &p, const LightArgs<R> &args, const CutTiles &ct, cudaStream_t s,
+                           bool sibling)
   {
     using L           = LightTile<MODE>;
     const size_t smem = L::template smem<R>();
@@ -122,9 +121,7 @@ namespace sint
       return e;
     const long long need   = (g.n_tiles + L::WARPS - 1) / L::WARPS;
     const long long blocks = need < grid_cap ? need : grid_cap;
-    k<<<dim3((unsigned)blocks), L::WARPS * 32, smem, s>>>(g, p, args, ct);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_dependent_if(sibling, k, dim3((unsigned)blocks), L::WARPS * 32, smem, s, g, p, args, ct);
   }
 
   // The one-kernel 2D cell loop (MODE: -1 = J v, 0..2 = residual).
@@ -200,16 +197,16 @@ namespace sint
 
   template <int DIM, bool TENS, typename R, bool ADV>
   cudaError_t launch_jvp_class(int K, const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
-                               const CutTiles &ct, const AdvData &adv, cudaStream_t s)
+                               const CutTiles &ct, const AdvData &adv, cudaStream_t s, bool sibling)
   {
     // the class without grains (c and mu only, the bulk of a packing's vapour)
     if constexpr (DIM == 3 && !ADV)
       if (K == 0)
-        return launch_light<TENS, R, -1>(g, p, LightArgs<R>{lin, src, {}, dst, partial}, ct, s);
+        return launch_light<TENS, R, -1>(g, p, LightArgs<R>{lin, src, {}, dst, partial}, ct, s, sibling);
     if constexpr (DIM == 2 && std::is_same_v<R, float> && !ADV)
       if (K == 0) // on tile pairs
-        return launch_jvp_pair_g<DIM, 0, TENS, true>(g, p, lin, src, dst, partial, s, ct);
-#define SINT_CALL(GG) launch_jvp_g<DIM, GG, TENS, R, true, ADV>(g, p, lin, src, dst, partial, ct, adv, s)
+        return launch_jvp_pair_g<DIM, 0, TENS, true>(g, p, lin, src, dst, partial, s, ct, sibling);
+#define SINT_CALL(GG) launch_jvp_g<DIM, GG, TENS, R, true, ADV>(g, p, lin, src, dst, partial, ct, adv, s, sibling)
     SINT_CLASS_SWITCH(K, SINT_CALL)
 #undef SINT_CALL
   }
@@ -242,9 +239,11 @@ namespace sint
   {
     if (cut)
       {
-        for (int K = 0; K <= G; ++K)
+        // the classes of many grains have few tiles and a long time per tile:
+        // launched first, they run beside the light ones (siblings_begin)
+        for (int K = G; K >= 0; --K)
           if (const cudaError_t e =
-                launch_jvp_class<DIM, TENS, R, ADV>(K, g, p, lin, src, dst, partial, *cut, adv, s))
+                launch_jvp_class<DIM, TENS, R, ADV>(K, g, p, lin, src, dst, partial, *cut, adv, s, K < G))
             return e;
         return cudaSuccess;
       }
@@ -284,7 +283,7 @@ namespace sint
   template <int DIM, bool TENS, bool CUT, int WTD, bool ADV>
   cudaError_t launch_residual_w(int G, const Grid &g, const Phys &p, const double *src, const double *const *hist,
                                 double *dst, double *partial, const CutTiles &ct, const AdvData &adv,
-                                cudaStream_t s)
+                                cudaStream_t s, bool sibling)
   {
     if constexpr (CUT)
       {
@@ -294,9 +293,9 @@ namespace sint
               LightArgs<double> args{src, nullptr, {}, dst, partial};
               for (int i = 0; WTD == 2 && i < p.order; ++i)
                 args.h[i] = hist[i];
-              return launch_light<TENS, double, WTD>(g, p, args, ct, s);
+              return launch_light<TENS, double, WTD>(g, p, args, ct, s, sibling);
             }
-#define SINT_CALL(GG) launch_residual_g<DIM, GG, TENS, WTD, true, ADV>(g, p, src, hist, dst, partial, ct, adv, s)
+#define SINT_CALL(GG) launch_residual_g<DIM, GG, TENS, WTD, true, ADV>(g, p, src, hist, dst, partial, ct, adv, s, sibling)
         SINT_CLASS_SWITCH(G, SINT_CALL)
 #undef SINT_CALL
       }
@@ -311,13 +310,13 @@ namespace sint
   template <int DIM, bool TENS, bool CUT, bool ADV>
   cudaError_t launch_residual_c(int G, int wtd, const Grid &g, const Phys &p, const double *src,
                                 const double *const *hist, double *dst, double *partial, const CutTiles &ct,
-                                const AdvData &adv, cudaStream_t s)
+                                const AdvData &adv, cudaStream_t s, bool sibling = false)
   {
     if (wtd == 0)
-      return launch_residual_w<DIM, TENS, CUT, 0, ADV>(G, g, p, src, hist, dst, partial, ct, adv, s);
+      return launch_residual_w<DIM, TENS, CUT, 0, ADV>(G, g, p, src, hist, dst, partial, ct, adv, s, sibling);
     if (wtd == 1)
-      return launch_residual_w<DIM, TENS, CUT, 1, ADV>(G, g, p, src, hist, dst, partial, ct, adv, s);
-    return launch_residual_w<DIM, TENS, CUT, 2, ADV>(G, g, p, src, hist, dst, partial, ct, adv, s);
+      return launch_residual_w<DIM, TENS, CUT, 1, ADV>(G, g, p, src, hist, dst, partial, ct, adv, s, sibling);
+    return launch_residual_w<DIM, TENS, CUT, 2, ADV>(G, g, p, src, hist, dst, partial, ct, adv, s, sibling);
   }
 
   template <int DIM, bool TENS, bool ADV>
@@ -327,9 +326,9 @@ namespace sint
   {
     if (cut)
       {
-        for (int K = 0; K <= G; ++K)
+        for (int K = G; K >= 0; --K) // as the Jacobian product
           if (const cudaError_t e =
-                launch_residual_c<DIM, TENS, true, ADV>(K, wtd, g, p, src, hist, dst, partial, *cut, adv, s))
+                launch_residual_c<DIM, TENS, true, ADV>(K, wtd, g, p, src, hist, dst, partial, *cut, adv, s, K < G))
             return e;
         return cudaSuccess;
       }

@@ -94,6 +94,7 @@ namespace sint
     constexpr bool JVP  = L::JVP;
     constexpr int  S    = L::SLOTS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    siblings_begin();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     R        *buf  = reinterpret_cast<R *>(smem_raw) + warp * (L::NBUF * L::BOX + L::KSZ);
     R        *K    = buf + L::NBUF * L::BOX;
@@ -379,5 +380,6 @@ namespace sint
       }
     if constexpr (JVP)
       cp_async_wait<0>();
+    siblings_end();
   }
 } // namespace sint
