@@ -1219,6 +1219,45 @@ namespace sint
     const NodePlan<DIM>      np(g);
     const long long          i0 = CUT ? (long long)ct.range[G] : 0;
     const long long          i1 = CUT ? (long long)ct.range[G + 1] : g.n_tiles;
+    // The next tile's nodal values (this thread's box node, every NG-th
+    // component) wait in registers while this tile's sums are stored: the
+    // history is combined with arithmetic, so cp.async cannot stage it.
+    constexpr int NV = (C + T::NG - 1) / T::NG;
+    R             rv[NV], rh[WTD == 2 ? NV : 1][3];
+    auto          load = [&](long long idx) {
+      if (idx >= i1 || !np.active)
+        return;
+      const unsigned long long gl   = CUT ? ct.tile_grains[idx] : 0ull;
+      const TileCoord          tc   = tile_coord_of<DIM>(g, CUT ? (long long)ct.tiles[idx] : idx);
+      // in an interior tile the box node exists and reads itself
+      bool      inside = true;
+      long long lidx   = tile_node0(g, tc) + np.off;
+      if (!tile_interior<DIM>(g, tc))
+        {
+          const BoxNode<DIM> bn(g, tc);
+          inside = bn.inside;
+          lidx   = bn.lidx;
+        }
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+        {
+          const int  comp = np.grp + n * T::NG;
+          const bool on   = inside && comp < C;
+          const long long off = on ? (CUT ? comp_of(comp, gl) : comp) * g.ld + lidx : 0;
+          rv[n]               = on ? src[off] : R(0);
+          if (on && ph.hooks.perturb) // the residual's perturbation hook: src + a x
+            rv[n] += ph.hooks.perturb_scale * ph.hooks.perturb[off];
+          if constexpr (WTD == 2)
+            {
+              // mu has no history
+              const bool h = on && comp != 1;
+              rh[n][0]     = h ? h0[off] : R(0);
+              rh[n][1]     = h && ph.order > 1 ? h1[off] : R(0);
+              rh[n][2]     = h && ph.order > 2 ? h2[off] : R(0);
+            }
+        }
+    };
+    load(i0 + blockIdx.x);
     for (long long idx = i0 + blockIdx.x; idx < i1; idx += gridDim.x)
       {
         const long long          tile = CUT ? (long long)ct.tiles[idx] : idx;
@@ -1228,38 +1267,24 @@ namespace sint
         const bool               interior = tile_interior<DIM>(g, tc);
         const long long          node0    = tile_node0(g, tc);
         const unsigned m = CUT ? local_mask<G>(cell_mask<DIM>(ct.cell_mask, g, tc, threadIdx.x % T::CELLS), gl) : ~0u;
-        // this thread's box node: in an interior tile it exists and reads itself
-        bool      inside = true;
-        long long lidx   = node0 + np.off;
-        if (!interior)
-          {
-            const BoxNode<DIM> bn(g, tc);
-            inside = bn.inside;
-            lidx   = bn.lidx;
-          }
         if (np.active)
-          for (int comp = np.grp; comp < C; comp += T::NG)
+#pragma unroll
+          for (int n = 0; n < NV; ++n)
             {
-              R v = R(0), hv = R(0);
-              if (inside)
-                {
-                  const long long off = (CUT ? comp_of(comp, gl) : comp) * g.ld + lidx;
-                  v                   = src[off];
-                  if (ph.hooks.perturb) // the residual's perturbation hook: src + a x
-                    v = src[off] + ph.hooks.perturb_scale * ph.hooks.perturb[off];
-                  // sum_i w_{i+1} u_old_i at the nodes (generic.h:947-966); mu has no history
-                  if (WTD == 2 && comp != 1)
-                    {
-                      hv = h0[off] * ph.w_hist[0];
-                      if (ph.order > 1)
-                        hv += h1[off] * ph.w_hist[1];
-                      if (ph.order > 2)
-                        hv += h2[off] * ph.w_hist[2];
-                    }
-                }
-              s_u[comp * T::BOXS + np.sb] = v;
+              const int comp = np.grp + n * T::NG;
+              if (comp >= C)
+                break;
+              s_u[comp * T::BOXS + np.sb] = rv[n];
+              // sum_i w_{i+1} u_old_i at the nodes (generic.h:947-966)
               if constexpr (WTD == 2)
-                s_h[comp * T::BOXS + np.sb] = hv;
+                {
+                  R hv = rh[n][0] * ph.w_hist[0];
+                  if (ph.order > 1)
+                    hv += rh[n][1] * ph.w_hist[1];
+                  if (ph.order > 2)
+                    hv += rh[n][2] * ph.w_hist[2];
+                  s_h[comp * T::BOXS + np.sb] = hv;
+                }
             }
         if constexpr (ADV)
           adv_stage<DIM, G, R, CUT>(adv, g, tc, gl, A_vel, A_has);
@@ -1278,6 +1303,7 @@ namespace sint
         __syncthreads();
         phase_integrate<DIM, G, FM, R, CUT, ADV>(p, g, k, tc, P, s_u, K, m, A_vel, A_has);
         __syncthreads();
+        load(idx + gridDim.x);
         if (interior)
           sum_and_store_interior<DIM>(K, C, g, tc.linear, np, node0, dst, partial, gl, CUT, ct.c_all, tm, &ph.hooks);
         else
