@@ -8,15 +8,21 @@
 // 27 taps, a second input, the bias, a broadcast addend and the leaky ReLU in
 // one pass: every output is written once, the input tile once staged.
 //
-// Block: 32 (x) x 8 (y) threads; each thread owns a column of ZB consecutive
-// output slices at its (x, y) for all COUT output channels (ZB x COUT FP32
-// accumulators).  Per input channel the block stages the (ZB + 2) x 10 x 34
-// input box (zero outside the window) and that channel's 27 x COUT weights
-// in shared memory with cp.async, double-buffered: the next channel's copies
-// are in flight while this one is computed.  A thread reads, per (dy, dx)
+// Block: 32 x 8 (x, y) threads, or 16 x 16 (conv3d_cover); each thread owns a
+// column of ZB consecutive output slices at its (x, y) for all COUT output
+// channels (ZB x COUT FP32 accumulators).  Per input channel the block stages
+// the (ZB + 2) x 10 x 34 (or 18 x 18) input box (zero outside the window) and
+// that channel's 27 x COUT weights in shared memory with cp.async,
+// double-buffered: the next channel's copies are in flight while this one is
+// computed.  A thread reads, per (dy, dx)
 // tap column, ZB + 2 input values and per dz the COUT weights (one broadcast
 // read serves the warp), and issues 3 ZB COUT fused multiply-adds, as packed
 // FP32 pairs of output channels (FFMA2) when COUT is a multiple of 4.
+//
+// Bound by issue and the FMA pipe (COUT 8, 96^3 window, 6 grains: 55 % of the
+// issue slots, a fifth of the warps resident at 128 registers); the addend and
+// the tile's overhang were what could be saved: 2237 -> 2083 us over the COUT 8
+// convolutions of that window, 3133 -> 3070 us for the whole guess.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -27,8 +33,7 @@ namespace sint
 {
   namespace
   {
-    constexpr int C3_TX = 32, C3_TY = 8, C3_THREADS = C3_TX * C3_TY;
-    constexpr int C3_PX = C3_TX + 3; // row pitch of the staged box (34 used)
+    constexpr int C3_THREADS = 256;
 
     struct Conv3dArgs
     {
@@ -67,9 +72,11 @@ namespace sint
       asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
     }
 
-    template <int COUT>
+    template <int COUT, int C3_TX>
     __global__ void __launch_bounds__(C3_THREADS, 2) conv3d_kernel(const Conv3dArgs a)
     {
+      constexpr int C3_TY = C3_THREADS / C3_TX;
+      constexpr int C3_PX = C3_TX == 32 ? 35 : C3_TX + 2; // row pitch of the staged box
       constexpr int ZB = conv3d_zb<COUT>();
       constexpr int BZ = ZB + 2, BY = C3_TY + 2, BX = C3_TX + 2;
       // double-buffered input box and weights of one input channel
@@ -85,9 +92,9 @@ namespace sint
       const int       D2 = a.D + 2;
       const int       nch = a.c[0] + a.c[1];
 
-      // stage input channel g (of x1 then x2) into buffer b: each warp copies
-      // whole box rows, lane l the row entries l and l + 32 (< BX); entries
-      // outside the window are zero-filled
+      // stage input channel g (of x1 then x2) into buffer b: a row of threads
+      // copies whole box rows, thread l the entries l and l + TX (< BX);
+      // entries outside the window are zero-filled
       auto stage = [&](int g, int b) {
         // selects, not a dynamic index into the parameter arrays (which would
         // copy them to local memory)
@@ -106,7 +113,7 @@ namespace sint
 #pragma unroll
             for (int h = 0; h < 2; ++h)
               {
-                const int bx = tx + 32 * h;
+                const int bx = tx + C3_TX * h;
                 if (bx < BX)
                   {
                     const int  xx = x0 - 1 + bx;
@@ -214,31 +221,45 @@ namespace sint
       const long long zs = (long long)a.cout * hw;
       float          *op = a.out + ((long long)s * D2 + z0) * zs + pix;
       const float    *ap = a.addend ? a.addend + ((long long)(s / a.addend_group) * D2 + z0) * zs + pix : nullptr;
+      constexpr int CE = COUT < 8 ? COUT : 8;
+      // the addends of CE channels are loaded together, and read-only so that they
+      // may go ahead of the stores before them: one at a time each load
+      // waited for its turn behind a store
 #pragma unroll
       for (int z = 0; z < ZB; ++z)
         {
           if (z0 + z > a.D)
             break;
 #pragma unroll
-          for (int co = 0; co < COUT; ++co)
+          for (int c0 = 0; c0 < COUT; c0 += CE)
             {
-              if (co >= a.cout)
-                break;
-              const long long o = z * zs + co * hw;
-              float           v;
-              if constexpr (PAIRS)
-                v = co & 1 ? acc2[z][co / 2].y : acc2[z][co / 2].x;
-              else
-                v = acc[z][co];
-              if (a.bias)
-                v += a.bias[co];
-              if (ap)
-                v += ap[o];
-              if (a.accumulate)
-                v += op[o];
-              if (a.leaky && v < 0.f)
-                v *= a.slope;
-              op[o] = v;
+              float add[CE];
+#pragma unroll
+              for (int c = 0; c < CE; ++c)
+                {
+                  const int co = c0 + c;
+                  add[c]       = ap && co < a.cout ? __ldg(ap + z * zs + co * hw) : 0.f;
+                  if (a.accumulate && co < a.cout)
+                    add[c] += op[z * zs + co * hw];
+                }
+#pragma unroll
+              for (int c = 0; c < CE; ++c)
+                {
+                  const int co = c0 + c;
+                  if (co >= a.cout)
+                    break;
+                  float v;
+                  if constexpr (PAIRS)
+                    v = co & 1 ? acc2[z][co / 2].y : acc2[z][co / 2].x;
+                  else
+                    v = acc[z][co];
+                  if (a.bias)
+                    v += __ldg(a.bias + co);
+                  v += add[c];
+                  if (a.leaky && v < 0.f)
+                    v *= a.slope;
+                  op[z * zs + co * hw] = v;
+                }
             }
         }
       // the depth padding of the output: slice 0 by the first z tile, D + 1 by the last
@@ -252,15 +273,35 @@ namespace sint
           }
     }
 
+    template <int COUT, int TX>
+    cudaError_t launch_conv3d_tile(const Conv3dArgs &a, cudaStream_t st)
+    {
+      constexpr int ZB = conv3d_zb<COUT>(), TY = C3_THREADS / TX;
+      const int     tiles_x = (a.W + TX - 1) / TX, tiles_y = (a.H + TY - 1) / TY;
+      const dim3    grid(unsigned(tiles_x * tiles_y), unsigned((a.D + ZB - 1) / ZB), unsigned(a.S));
+      conv3d_kernel<COUT, TX><<<grid, C3_THREADS, 0, st>>>(a);
+      count_launches(1);
+      return cudaGetLastError();
+    }
+    // threads of a TX-wide tiling of the window
+    inline long long conv3d_cover(const Conv3dArgs &a, int TX)
+    {
+      const int TY = C3_THREADS / TX;
+      return (long long)((a.W + TX - 1) / TX * TX) * ((a.H + TY - 1) / TY * TY);
+    }
+    // The packed instances are bound by their multiply-adds, those of the threads
+    // outside the window included: they take the tiling with less overhang (97 x
+    // 97 nodes: 112 x 112 against 128 x 104, 6 % fewer threads).  The others are
+    // bound by their shared-memory reads, where two box rows in a warp share
+    // banks: COUT 1 took 599 us in 16 x 16 tiles against 518 in 32 x 8 ones, COUT
+    // 2 181 against 171 (96^3 window, 6 grains), so they stay with 32 x 8.
     template <int COUT>
     cudaError_t launch_conv3d(const Conv3dArgs &a, cudaStream_t st)
     {
-      constexpr int ZB      = conv3d_zb<COUT>();
-      const int     tiles_x = (a.W + C3_TX - 1) / C3_TX, tiles_y = (a.H + C3_TY - 1) / C3_TY;
-      const dim3    grid(unsigned(tiles_x * tiles_y), unsigned((a.D + ZB - 1) / ZB), unsigned(a.S));
-      conv3d_kernel<COUT><<<grid, C3_THREADS, 0, st>>>(a);
-      count_launches(1);
-      return cudaGetLastError();
+      if constexpr (COUT % 4 == 0)
+        if (conv3d_cover(a, 16) < conv3d_cover(a, 32))
+          return launch_conv3d_tile<COUT, 16>(a, st);
+      return launch_conv3d_tile<COUT, 32>(a, st);
     }
   } // namespace
 } // namespace sint
@@ -275,7 +316,7 @@ int sint_nn_conv3d_f32(int S, int D, int H, int W, const float *x1, int c1, cons
 {
   if (S < 1 || D < 1 || H < 1 || W < 1 || !x1 || !w1 || c1 < 1 || c2 < 0 || (c2 > 0 && (!x2 || !w2)) || !out ||
       cout < 1 || cout > 32 || (addend && (addend_group < 1 || S % addend_group != 0)) ||
-      (long long)((W + C3_TX - 1) / C3_TX) * ((H + C3_TY - 1) / C3_TY) >= (1ll << 31) || S > 65535)
+      (long long)((W + 31) / 32) * ((H + 7) / 8) >= (1ll << 31) || S > 65535)
     {
       set_error("sint_nn_conv3d_f32: bad argument");
       return SINT_ERR_ARG;
