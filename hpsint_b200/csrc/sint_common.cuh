@@ -792,8 +792,8 @@ namespace sint
   // only when bit b of tile_mask[tile] is set.  Most shared nodes of a packing
   // lie between tiles without a relevant grain, so there one thread serves all
   // components: c and mu together, then a grain only where a sharing tile wrote
-  // it (256^3 cells, 12 components: 0.77 ms in
-  // groups of six components).
+  // it (256^3 cells, 12 components: 0.38 ms, 0.77 ms in groups of six
+  // components, 0.40 ms with a few loads of each component at a time).
   // epi (the residual's epilogue hook, nullptr for none): the combined sums
   // are stored as (sum - sub) * scale.
   template <int DIM, typename R, int CH, bool MASKED>

@@ -1063,19 +1063,19 @@ namespace sint
   }
 
   // -------------------------------------------------------------------------
-  // FP32 Jacobian-vector product of few grains on tile pairs.  sm_100 executes FP32 add,
-  // multiply and fused multiply-add on two values held in a 64-bit register
-  // pair with one instruction (FADD2 / FMUL2 / FFMA2); the FP32 product is
-  // bound by instruction issue, so the block computes tiles 2j and 2j + 1
-  // together: every shared-memory value is a pair (lane x of tile 2j, lane y
-  // of tile 2j + 1), phases 1-3 run once on F2 for both tiles, and the node
-  // sums are stored per lane.  Each lane rounds exactly as the scalar FP32
-  // arithmetic of the same expression does.  Full operator only (no grain
-  // cut-off, no advection: those keep jvp_kernel); shared memory and
+  // FP32 Jacobian-vector product of few grains on tile pairs.  sm_100 executes
+  // FP32 add, multiply and fused multiply-add on two values held in a 64-bit
+  // register pair with one instruction (FADD2 / FMUL2 / FFMA2); the FP32
+  // product is bound by instruction issue, so the block computes tiles 2j and
+  // 2j + 1 together: every shared-memory value is a pair (lane x of tile 2j,
+  // lane y of tile 2j + 1), phases 1-3 run once on F2 for both tiles, and the
+  // node sums are stored per lane.  Each lane rounds exactly as the scalar FP32
+  // arithmetic of the same expression does.  The full 3D operator without
+  // advection, up to four grains (launch_jvp_full says why); shared memory and
   // registers as the FP64 product.
-  // CUT (G = 0 only): the grain cut-off's class of tiles without a relevant
-  // grain, ct.tiles[ct.range[0] .. ct.range[1]), on c and mu; their owned
-  // nodes get zero grain rows, as jvp_kernel's class-0 instance writes them.
+  // CUT (2D, G = 0 only): the grain cut-off's class of tiles without a relevant
+  // grain, ct.tiles[ct.range[0] .. ct.range[1]), on c and mu; their owned nodes
+  // get zero grain rows.
   // Resident blocks per SM: as the FP64 product (pairs take the FP64 product's
   // registers), but three for the class without grains, whose pairs need
   // ~70 registers (four blocks would cap them at 64 and spill).

@@ -175,39 +175,22 @@ namespace sint
       default: return cudaErrorInvalidValue;                                                                      \
     }
 
-  // The same over the grain-count classes 0..12 of the grain cut-off.
-#define SINT_CLASS_SWITCH(K, CALL)                                                                                \
-  switch (K)                                                                                                      \
-    {                                                                                                             \
-      case 0: return CALL(0);                                                                                     \
-      case 1: return CALL(1);                                                                                     \
-      case 2: return CALL(2);                                                                                     \
-      case 3: return CALL(3);                                                                                     \
-      case 4: return CALL(4);                                                                                     \
-      case 5: return CALL(5);                                                                                     \
-      case 6: return CALL(6);                                                                                     \
-      case 7: return CALL(7);                                                                                     \
-      case 8: return CALL(8);                                                                                     \
-      case 9: return CALL(9);                                                                                     \
-      case 10: return CALL(10);                                                                                   \
-      case 11: return CALL(11);                                                                                   \
-      case 12: return CALL(12);                                                                                   \
-      default: return cudaErrorInvalidValue;                                                                      \
-    }
-
+  // G = the class of the grain cut-off (0..12 relevant grains)
   template <int DIM, bool TENS, typename R, bool ADV>
-  cudaError_t launch_jvp_class(int K, const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
+  cudaError_t launch_jvp_class(int G, const Grid &g, const Phys &p, const R *lin, const R *src, R *dst, R *partial,
                                const CutTiles &ct, const AdvData &adv, cudaStream_t s, bool sibling)
   {
-    // the class without grains (c and mu only, the bulk of a packing's vapour)
-    if constexpr (DIM == 3 && !ADV)
-      if (K == 0)
-        return launch_light<TENS, R, -1>(g, p, LightArgs<R>{lin, src, {}, dst, partial}, ct, s, sibling);
-    if constexpr (DIM == 2 && std::is_same_v<R, float> && !ADV)
-      if (K == 0) // on tile pairs
-        return launch_jvp_pair_g<DIM, 0, TENS, true>(g, p, lin, src, dst, partial, s, ct, sibling);
 #define SINT_CALL(GG) launch_jvp_g<DIM, GG, TENS, R, true, ADV>(g, p, lin, src, dst, partial, ct, adv, s, sibling)
-    SINT_CLASS_SWITCH(K, SINT_CALL)
+    if (G == 0) // without grains: c and mu only, the bulk of a packing's vapour
+      {
+        if constexpr (DIM == 3 && !ADV)
+          return launch_light<TENS, R, -1>(g, p, LightArgs<R>{lin, src, {}, dst, partial}, ct, s, sibling);
+        else if constexpr (std::is_same_v<R, float> && !ADV) // on tile pairs
+          return launch_jvp_pair_g<DIM, 0, TENS, true>(g, p, lin, src, dst, partial, s, ct, sibling);
+        else
+          return SINT_CALL(0);
+      }
+    SINT_G_SWITCH(SINT_CALL)
 #undef SINT_CALL
   }
 
@@ -287,16 +270,20 @@ namespace sint
   {
     if constexpr (CUT)
       {
-        if constexpr (DIM == 3 && !ADV)
-          if (G == 0)
-            {
-              LightArgs<double> args{src, nullptr, {}, dst, partial};
-              for (int i = 0; WTD == 2 && i < p.order; ++i)
-                args.h[i] = hist[i];
-              return launch_light<TENS, double, WTD>(g, p, args, ct, s, sibling);
-            }
 #define SINT_CALL(GG) launch_residual_g<DIM, GG, TENS, WTD, true, ADV>(g, p, src, hist, dst, partial, ct, adv, s, sibling)
-        SINT_CLASS_SWITCH(G, SINT_CALL)
+        if (G == 0)
+          {
+            if constexpr (DIM == 3 && !ADV)
+              {
+                LightArgs<double> args{src, nullptr, {}, dst, partial};
+                for (int i = 0; WTD == 2 && i < p.order; ++i)
+                  args.h[i] = hist[i];
+                return launch_light<TENS, double, WTD>(g, p, args, ct, s, sibling);
+              }
+            else
+              return SINT_CALL(0);
+          }
+        SINT_G_SWITCH(SINT_CALL)
 #undef SINT_CALL
       }
     else
