@@ -19,10 +19,14 @@
 // read serves the warp), and issues 3 ZB COUT fused multiply-adds, as packed
 // FP32 pairs of output channels (FFMA2) when COUT is a multiple of 4.
 //
-// Bound by issue and the FMA pipe (COUT 8, 96^3 window, 6 grains: 55 % of the
-// issue slots, a fifth of the warps resident at 128 registers); the addend and
-// the tile's overhang were what could be saved: 2237 -> 2083 us over the COUT 8
-// convolutions of that window, 3133 -> 3070 us for the whole guess.
+// Bound by issue and the FMA pipe, so what is not a multiply-add is kept out of
+// the channel loop: a thread stages the same one or two (x, y) entries of every
+// slice, its bounds test and offset serve the whole column, and entries outside
+// the window are zeroed once for all channels.  (Row by row with a test per
+// entry, staging was a fifth of the instructions at COUT 8 and almost half at
+// COUT 1.)  96^3 window, 6 grains, whole guess: 3133 us with 32 x 8 tiles, rows
+// and one addend at a time, 3070 us with tiles and addends as here, 2596 us with
+// the staging by columns.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -92,9 +96,20 @@ namespace sint
       const int       D2 = a.D + 2;
       const int       nch = a.c[0] + a.c[1];
 
-      // stage input channel g (of x1 then x2) into buffer b: a row of threads
-      // copies whole box rows, thread l the entries l and l + TX (< BX);
-      // entries outside the window are zero-filled
+      // a thread copies the same one or two entries of every slice of the box
+      constexpr int NE = (BY * BX + C3_THREADS - 1) / C3_THREADS;
+      // box entries outside the window are zero for all channels
+      if (x0 == 0 || y0 == 0 || z0 == 1 || x0 + C3_TX >= a.W || y0 + C3_TY >= a.H || z0 + ZB > a.D)
+        {
+          float *z = &s_in[0][0][0][0];
+          for (int i = threadIdx.x; i < 2 * BZ * BY * C3_PX; i += C3_THREADS)
+            z[i] = 0.f;
+          __syncthreads();
+        }
+      // slices of the box inside the window: bz0 <= bz < bz1
+      const int bz0 = z0 == 1 ? 1 : 0, bz1 = min(BZ, a.D + 2 - z0);
+
+      // stage input channel g (of x1 then x2) into buffer b
       auto stage = [&](int g, int b) {
         // selects, not a dynamic index into the parameter arrays (which would
         // copy them to local memory)
@@ -103,23 +118,22 @@ namespace sint
         const int    ck  = k ? a.c[1] : a.c[0];
         const float *xk  = k ? a.x[1] : a.x[0];
         const float *wk  = k ? a.w[1] : a.w[0];
-        const float *src = xk + (long long)s * D2 * ck * hw + (long long)ci * hw;
-        for (int row = ty; row < BZ * BY; row += C3_TY)
-          {
-            const int  bz = row / BY, by = row % BY;
-            const int  zz = z0 - 1 + bz, yy = y0 - 1 + by;
-            const bool rv = zz >= 1 && zz <= a.D && yy >= 0 && yy < a.H;
-            const float *rp = src + (long long)zz * ck * hw + (long long)yy * a.W;
+        const long long zstep = ck * hw;
+        const float    *src   = xk + ((long long)s * D2 + z0 - 1) * zstep + (long long)ci * hw;
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < NE; ++h)
+          {
+            const int i  = threadIdx.x + C3_THREADS * h;
+            const int by = i / BX, bx = i % BX;
+            const int yy = y0 - 1 + by, xx = x0 - 1 + bx;
+            if (by < BY && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W)
               {
-                const int bx = tx + C3_TX * h;
-                if (bx < BX)
-                  {
-                    const int  xx = x0 - 1 + bx;
-                    const bool v  = rv && xx >= 0 && xx < a.W;
-                    cp_async4(&s_in[b][bz][by][bx], v ? rp + xx : a.x[0], v);
-                  }
+                const float *sp = src + (long long)yy * a.W + xx;
+                float       *dp = &s_in[b][0][by][bx];
+#pragma unroll
+                for (int bz = 0; bz < BZ; ++bz)
+                  if (bz >= bz0 && bz < bz1)
+                    cp_async4(dp + bz * (BY * C3_PX), sp + bz * zstep, true);
               }
           }
         for (int i = threadIdx.x; i < 27 * COUT; i += C3_THREADS)
