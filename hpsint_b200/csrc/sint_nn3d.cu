@@ -8,13 +8,14 @@
 // 27 taps, a second input, the bias, a broadcast addend and the leaky ReLU in
 // one pass: every output is written once, the input tile once staged.
 //
-// Block: 32 x 8 (x, y) threads, or 16 x 16 (conv3d_cover); each thread owns a
-// column of ZB consecutive output slices at its (x, y) for all COUT output
-// channels (ZB x COUT FP32 accumulators).  Per input channel the block stages
-// the (ZB + 2) x 10 x 34 (or 18 x 18) input box (zero outside the window) and
-// that channel's 27 x COUT weights in shared memory with cp.async,
-// double-buffered: the next channel's copies are in flight while this one is
-// computed.  A thread reads, per (dy, dx)
+// Block: 256 threads on a tile of the (x, y) plane whose width (16 to 32) is
+// chosen for the window (launch_conv3d); each thread owns a column of ZB
+// consecutive output slices at its (x, y) for all COUT output channels (ZB x
+// COUT FP32 accumulators).  Per input channel the block stages the ZB + 2
+// slices of the tile with its halo (zero outside the window) and that
+// channel's 27 x COUT weights in shared memory with cp.async, double-buffered:
+// the next channel's copies are in flight while this one is computed.  A
+// thread reads, per (dy, dx)
 // tap column, ZB + 2 input values and per dz the COUT weights (one broadcast
 // read serves the warp), and issues 3 ZB COUT fused multiply-adds, as packed
 // FP32 pairs of output channels (FFMA2) when COUT is a multiple of 4.
@@ -25,8 +26,10 @@
 // the window are zeroed once for all channels.  (Row by row with a test per
 // entry, staging was a fifth of the instructions at COUT 8 and almost half at
 // COUT 1.)  96^3 window, 6 grains, whole guess: 3133 us with 32 x 8 tiles, rows
-// and one addend at a time, 3070 us with tiles and addends as here, 2596 us with
-// the staging by columns.
+// and one addend at a time; 3070 us with 16 x 16 tiles where they fit better and
+// the addends as here; 2596 us with the staging by columns; 2300 us with the
+// width chosen for the window.
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -38,6 +41,7 @@ namespace sint
   namespace
   {
     constexpr int C3_THREADS = 256;
+    constexpr int C3_BOX     = 340; // largest (x, y) box of a tile with its halo
 
     struct Conv3dArgs
     {
@@ -53,6 +57,8 @@ namespace sint
       float       *out; // [S][D + 2][cout][H][W]
       int          cout;
       int          accumulate;
+      int          tx, ty;   // tile of the (x, y) plane, tx * ty <= C3_THREADS
+      unsigned     div_bx;   // ceil(2^16 / (tx + 2))
     };
 
     // output slices per thread: ZB x COUT accumulators stay within 64 registers,
@@ -76,33 +82,34 @@ namespace sint
       asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
     }
 
-    template <int COUT, int C3_TX>
-    __global__ void __launch_bounds__(C3_THREADS, 2) conv3d_kernel(const Conv3dArgs a)
+    template <int COUT>
+    __global__ void __launch_bounds__(C3_THREADS, COUT <= 2 ? 3 : 2) conv3d_kernel(const Conv3dArgs a)
     {
-      constexpr int C3_TY = C3_THREADS / C3_TX;
-      constexpr int C3_PX = C3_TX == 32 ? 35 : C3_TX + 2; // row pitch of the staged box
       constexpr int ZB = conv3d_zb<COUT>();
-      constexpr int BZ = ZB + 2, BY = C3_TY + 2, BX = C3_TX + 2;
+      constexpr int BZ = ZB + 2;
+      const int     BX = a.tx + 2, box = BX * (a.ty + 2);
       // double-buffered input box and weights of one input channel
-      __shared__ float s_in[2][BZ][BY][C3_PX];
+      __shared__ float s_in[2][BZ][C3_BOX]; // row pitch BX
       __shared__ __align__(16) float s_w[2][27][COUT];
 
-      const int tiles_x = (a.W + C3_TX - 1) / C3_TX;
-      const int x0 = (blockIdx.x % tiles_x) * C3_TX, y0 = (blockIdx.x / tiles_x) * C3_TY;
+      const int tiles_x = (a.W + a.tx - 1) / a.tx;
+      const int x0 = (blockIdx.x % tiles_x) * a.tx, y0 = (blockIdx.x / tiles_x) * a.ty;
       const int z0 = 1 + blockIdx.y * ZB; // first output slice (window slice index)
       const int s  = blockIdx.z;
-      const int tx = threadIdx.x % C3_TX, ty = threadIdx.x / C3_TX;
+      // threads beyond the tile compute its first node again and store nothing
+      const bool idle = threadIdx.x >= a.tx * a.ty;
+      const int  ty = idle ? 0 : threadIdx.x / a.tx, tx = idle ? 0 : threadIdx.x - ty * a.tx;
       const long long hw = (long long)a.H * a.W;
       const int       D2 = a.D + 2;
       const int       nch = a.c[0] + a.c[1];
 
       // a thread copies the same one or two entries of every slice of the box
-      constexpr int NE = (BY * BX + C3_THREADS - 1) / C3_THREADS;
+      constexpr int NE = (C3_BOX + C3_THREADS - 1) / C3_THREADS;
       // box entries outside the window are zero for all channels
-      if (x0 == 0 || y0 == 0 || z0 == 1 || x0 + C3_TX >= a.W || y0 + C3_TY >= a.H || z0 + ZB > a.D)
+      if (x0 == 0 || y0 == 0 || z0 == 1 || x0 + a.tx >= a.W || y0 + a.ty >= a.H || z0 + ZB > a.D)
         {
-          float *z = &s_in[0][0][0][0];
-          for (int i = threadIdx.x; i < 2 * BZ * BY * C3_PX; i += C3_THREADS)
+          float *z = &s_in[0][0][0];
+          for (int i = threadIdx.x; i < 2 * BZ * C3_BOX; i += C3_THREADS)
             z[i] = 0.f;
           __syncthreads();
         }
@@ -124,16 +131,16 @@ namespace sint
         for (int h = 0; h < NE; ++h)
           {
             const int i  = threadIdx.x + C3_THREADS * h;
-            const int by = i / BX, bx = i % BX;
+            const int by = int((unsigned(i) * a.div_bx) >> 16), bx = i - by * BX; // exact: i * BX < 2^16
             const int yy = y0 - 1 + by, xx = x0 - 1 + bx;
-            if (by < BY && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W)
+            if (i < box && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W)
               {
                 const float *sp = src + (long long)yy * a.W + xx;
-                float       *dp = &s_in[b][0][by][bx];
+                float       *dp = &s_in[b][0][i];
 #pragma unroll
                 for (int bz = 0; bz < BZ; ++bz)
                   if (bz >= bz0 && bz < bz1)
-                    cp_async4(dp + bz * (BY * C3_PX), sp + bz * zstep, true);
+                    cp_async4(dp + bz * C3_BOX, sp + bz * zstep, true);
               }
           }
         for (int i = threadIdx.x; i < 27 * COUT; i += C3_THREADS)
@@ -159,6 +166,7 @@ namespace sint
               acc[z][co] = 0.f;
           }
 
+      const int at = ty * BX + tx; // first tap's entry of the thread's column
       stage(0, 0);
       cp_async_commit_group();
       for (int g = 0; g < nch; ++g)
@@ -177,7 +185,7 @@ namespace sint
                 float col[BZ];
 #pragma unroll
                 for (int z = 0; z < BZ; ++z)
-                  col[z] = s_in[b][z][ty + dy][tx + dx];
+                  col[z] = s_in[b][z][at + dy * BX + dx];
                 if constexpr (COUT % 4 == 0)
                   {
                     // packed FP32 pairs: two output channels per FFMA2 (each
@@ -228,7 +236,7 @@ namespace sint
       cp_async_wait_group<0>();
 
       const int x = x0 + tx, y = y0 + ty;
-      if (x >= a.W || y >= a.H)
+      if (idle || x >= a.W || y >= a.H)
         return;
       const long long pix = (long long)y * a.W + x;
       // slice z0, channel 0 of this thread's output and addend columns
@@ -287,35 +295,37 @@ namespace sint
           }
     }
 
-    template <int COUT, int TX>
-    cudaError_t launch_conv3d_tile(const Conv3dArgs &a, cudaStream_t st)
+    // Tiles of the window when they are tx wide: as many rows as the threads
+    // and the staged box allow.  The width with the fewest tiles is taken: the
+    // multiply-adds of threads outside the window are what a kernel bound by its
+    // arithmetic can save (97 x 97 nodes: 40 tiles of 25 x 10, 49 of 16 x 16, 52
+    // of 32 x 8; 33 x 33: 6 of 23 x 11, 9, 10).  4 windows of 48 x 97 x
+    // 97, against tiles of 32 x 8 (COUT 1, 2) or 16 x 16: COUT 2 103 -> 90 us, 4
+    // 149 -> 136, 8 218 -> 205, 16 781 -> 621, 32 5454 -> 4458; COUT 1, bound by
+    // its shared-memory reads, where a warp on two rows meets some banks twice,
+    // 77 -> 78.  Where 32 x 8 fits (2 of 24 x 64 x 64) the pitch in a register
+    // instead of a constant costs up to 2 us of 25 to 39 at COUT 2 and 8 and
+    // nothing at 1, 4, 16 and 32.
+    inline int conv3d_rows(int tx) { return std::min(C3_THREADS / tx, C3_BOX / (tx + 2) - 2); }
+    inline long long conv3d_tiles(const Conv3dArgs &a, int tx)
     {
-      constexpr int ZB = conv3d_zb<COUT>(), TY = C3_THREADS / TX;
-      const int     tiles_x = (a.W + TX - 1) / TX, tiles_y = (a.H + TY - 1) / TY;
-      const dim3    grid(unsigned(tiles_x * tiles_y), unsigned((a.D + ZB - 1) / ZB), unsigned(a.S));
-      conv3d_kernel<COUT, TX><<<grid, C3_THREADS, 0, st>>>(a);
+      const int ty = conv3d_rows(tx);
+      return (long long)((a.W + tx - 1) / tx) * ((a.H + ty - 1) / ty);
+    }
+    template <int COUT>
+    cudaError_t launch_conv3d(Conv3dArgs a, cudaStream_t st)
+    {
+      constexpr int ZB = conv3d_zb<COUT>();
+      a.tx             = 32;
+      for (int tx = 31; tx >= 16; --tx)
+        if (conv3d_tiles(a, tx) < conv3d_tiles(a, a.tx))
+          a.tx = tx;
+      a.ty     = conv3d_rows(a.tx);
+      a.div_bx = (65536 + a.tx + 1) / (a.tx + 2);
+      const dim3 grid(unsigned(conv3d_tiles(a, a.tx)), unsigned((a.D + ZB - 1) / ZB), unsigned(a.S));
+      conv3d_kernel<COUT><<<grid, C3_THREADS, 0, st>>>(a);
       count_launches(1);
       return cudaGetLastError();
-    }
-    // threads of a TX-wide tiling of the window
-    inline long long conv3d_cover(const Conv3dArgs &a, int TX)
-    {
-      const int TY = C3_THREADS / TX;
-      return (long long)((a.W + TX - 1) / TX * TX) * ((a.H + TY - 1) / TY * TY);
-    }
-    // The packed instances are bound by their multiply-adds, those of the threads
-    // outside the window included: they take the tiling with less overhang (97 x
-    // 97 nodes: 112 x 112 against 128 x 104, 6 % fewer threads).  The others are
-    // bound by their shared-memory reads, where two box rows in a warp share
-    // banks: COUT 1 took 599 us in 16 x 16 tiles against 518 in 32 x 8 ones, COUT
-    // 2 181 against 171 (96^3 window, 6 grains), so they stay with 32 x 8.
-    template <int COUT>
-    cudaError_t launch_conv3d(const Conv3dArgs &a, cudaStream_t st)
-    {
-      if constexpr (COUT % 4 == 0)
-        if (conv3d_cover(a, 16) < conv3d_cover(a, 32))
-          return launch_conv3d_tile<COUT, 16>(a, st);
-      return launch_conv3d_tile<COUT, 32>(a, st);
     }
   } // namespace
 } // namespace sint

@@ -1,6 +1,6 @@
-"""Tilings of the one-pass 3x3x3 convolution of the 3D guess (sint_nn3d.cu): 16
-x 16 blocks where they overhang the window less than 32 x 8 ones, for output
-channels in packed pairs; the others keep 32 x 8."""
+"""Tilings of the one-pass 3x3x3 convolution of the 3D guess (sint_nn3d.cu): the
+tile width is chosen for the window, with idle threads in tiles of fewer than
+256 nodes."""
 import numpy as np
 import pytest
 from oracle import predictor_ref as R
@@ -17,8 +17,10 @@ def padded(a):
     return t
 
 
-# windows just below, at and above the edges of both tilings
-@pytest.mark.parametrize("H,W", [(15, 15), (16, 16), (17, 48), (16, 33), (31, 15), (33, 33), (8, 32), (1, 1)])
+# windows just below, at and above the edges of 16 x 16 and 32 x 8 tiles, and
+# widths in between (25 x 25: tiles of 28 x 9, 49 x 70: 25 x 10)
+@pytest.mark.parametrize("H,W", [(15, 15), (16, 16), (17, 48), (16, 33), (31, 15), (33, 33), (8, 32), (1, 1), (25, 25),
+                                 (49, 70), (5, 97)])
 @pytest.mark.parametrize("cout", [1, 2, 3, 5, 16, 17])
 def test_conv3d_tilings(H, W, cout):
     from hpsint_b200 import predictor as P
