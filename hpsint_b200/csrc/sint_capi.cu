@@ -662,7 +662,8 @@ int sint_precond_setup(sint_ctx *c, sint_stream_t stream)
       set_error("sint_precond_setup: no linearisation point set");
       return SINT_ERR_NOT_READY;
     }
-  c->has_ch = false;
+  // a set-up that fails part way leaves neither kind of block 0 complete
+  c->has_pc = c->has_ch = false;
   if (c->pc_kind == 1)
     {
       // the Cahn-Hilliard matrix, and from the same passes the grains' diagonal
