@@ -58,17 +58,25 @@ namespace sint
     int      blocks_x; // blocks per row of blocks
   };
 
-  // Resident blocks per SM the registers are shared out for: the FP64 point
-  // physics and row sums of more grains need 255 registers (two blocks);
-  // capped at 128 (four blocks) they spill.
-  template <int G, bool TENS, typename R>
+  // Resident blocks per SM the registers are shared out for.  Four blocks leave
+  // 128 registers a thread, and the point physics of more grains spill there
+  // (bytes stored per thread: FP32 J v tensorial from 28 for 7 grains to 536 for
+  // 12, scalar from 16 for 8 to 136 for 12; FP64 tensorial 56 for 3, scalar 80
+  // and 152 for 4 and 5).  Spills cost most on meshes of about one block per
+  // SM, where nothing hides them.  Device time in us of the FP32 tensorial J v,
+  // four / three blocks: 128 x 128 cells 14.7 / 11.5 (8 grains), 27.9 / 22.2
+  // (12), where the tiled kernels take 14.8 and 26.9; 512 x 512 64.8 / 62.6 and
+  // 140.8 / 126.8; 7 grains 1024 x 1024 202 / 205.  Of the FP64 tensorial J v
+  // of 3 grains, four / two blocks: 136 x 136 9.1 / 5.3 (tiled 8.7), 1024 x
+  // 1024 134.7 / 132.1; its residual 124.1 / 129.7 there, so it keeps four.
+  template <int G, bool TENS, typename R, int MODE>
   constexpr int fused2d_blocks()
   {
-    return sizeof(R) == 4 || G <= (TENS ? 3 : 5) ? 4 : 2;
+    return sizeof(R) == 4 ? (TENS && G >= 8 ? 3 : 4) : G <= (TENS ? (MODE < 0 ? 2 : 3) : 5) ? 4 : 2;
   }
 
   template <int G, bool TENS, typename R, int MODE>
-  __global__ void __launch_bounds__(Fused2D<G, MODE>::THREADS, fused2d_blocks<G, TENS, R>())
+  __global__ void __launch_bounds__(Fused2D<G, MODE>::THREADS, fused2d_blocks<G, TENS, R, MODE>())
     fused2d_kernel(const Grid g, const Phys ph, const Fused2DArgs<R> args)
   {
     using L = Fused2D<G, MODE>;

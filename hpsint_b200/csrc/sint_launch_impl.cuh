@@ -135,7 +135,7 @@ namespace sint
     int                ready = 0;
     if (const cudaError_t e = per_device(cache, ready, [&](int, int &v) {
           v = 1;
-          return prepare_smem(k, smem, fused2d_blocks<G, TENS, R>());
+          return prepare_smem(k, smem, fused2d_blocks<G, TENS, R, MODE>());
         }))
       return e;
     args.blocks_x          = (g.nn[0] + L::TX - 2) / (L::TX - 1);
