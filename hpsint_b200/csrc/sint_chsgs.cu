@@ -938,22 +938,13 @@ namespace sint
       const bool     first = fwd && colour == 0;
       const unsigned nb    = (unsigned)((cnt + T - 1) / T);
       const unsigned ac    = first ? (unsigned)((g.N + T * V - 1) / (T * V)) : 0u;
-      cudaLaunchConfig_t    cfg{};
-      cudaLaunchAttribute   attr{};
-      attr.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr.val.programmaticStreamSerializationAllowed = 1;
-      cfg.gridDim                                     = dim3(nb + ac);
-      cfg.blockDim                                    = dim3(T);
-      cfg.stream                                      = s;
-      cfg.attrs                                       = &attr;
-      cfg.numAttrs                                    = first ? 0 : 1;
-      auto go = [&](auto k) { return cudaLaunchKernelEx(&cfg, k, g, colour, cl, A, r, z, nb, c->G, ac_inv); };
+      auto           go = [&](auto k) {
+        return launch_dependent_if(!first, k, dim3(nb + ac), dim3(T), 0, s, g, colour, cl, A, r, z, nb, c->G, ac_inv);
+      };
       // the rows of one wave of blocks at the registers all runs take
-      const bool        all = cnt <= (sizeof(R) == 4 ? SGS_WAVE_F32 : SGS_WAVE_F64);
-      const cudaError_t e   = fwd ? (all ? go(ch_sgs_kernel<DIM, R, true, DIM>) : go(ch_sgs_kernel<DIM, R, true, 2>)) :
-                                    (all ? go(ch_sgs_kernel<DIM, R, false, DIM>) : go(ch_sgs_kernel<DIM, R, false, 2>));
-      count_launches(1);
-      return e;
+      const bool all = cnt <= (sizeof(R) == 4 ? SGS_WAVE_F32 : SGS_WAVE_F64);
+      return fwd ? (all ? go(ch_sgs_kernel<DIM, R, true, DIM>) : go(ch_sgs_kernel<DIM, R, true, 2>)) :
+                   (all ? go(ch_sgs_kernel<DIM, R, false, DIM>) : go(ch_sgs_kernel<DIM, R, false, 2>));
     };
     for (int col = 0; col < NCOL; ++col)
       if (cudaError_t e = launch(col, true))

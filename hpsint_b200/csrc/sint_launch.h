@@ -129,7 +129,10 @@ namespace sint
     cfg.attrs                                       = &attr;
     cfg.numAttrs                                    = dependent ? 1 : 0;
     count_launches(1);
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+    if (e != cudaSuccess)
+      cudaGetLastError(); // reported by this call: the next one must not find it
+    return e;
   }
   template <typename... Params, typename... Args>
   inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,

@@ -54,3 +54,28 @@ def test_a_failed_set_up_leaves_no_preconditioner(block_0):
     pc.do_update()
     pc.vmult(z, r)
     assert torch.equal(z, want)
+
+
+@pytest.mark.parametrize("call", ["jvp_2d", "jvp_3d", "dot", "precond_block_jacobi", "precond_ch_gauss_seidel"])
+def test_a_failed_launch_fails_its_own_call_only(call):
+    import hpsint_b200 as hb
+    from hpsint_b200 import _lib as L
+    dim, cells, G = (3, (6, 5, 4), 2) if call == "jvp_3d" else (2, (9, 7), 2)
+    op = hb.SinteringOperatorGeneric(hb.Mesh(dim, cells), hb.Params(G))
+    op.set_time_weights(1e3, [-1e3], 1.0)
+    u = op.to_device(random_state(dim, cells, G, seed=3))
+    op.fill_quadrature_point_values(u)
+    z, h, lib = op.initialize_dof_vector(), op._h, L.lib()
+    if call.startswith("precond"):
+        pc = hb.BlockPreconditioner2(op, block_0=call[len("precond_"):])
+        pc.do_update()
+    with refusing_stream() as s:
+        if call == "dot":
+            rc = lib.sint_vec_dot_f64(h, u.numel(), u.data_ptr(), u.data_ptr(), z.data_ptr(), s)
+        else:
+            f = lib.sint_jvp_f64 if call.startswith("jvp") else lib.sint_precond_apply_f64
+            rc = f(h, z.data_ptr(), u.data_ptr(), s)
+        assert L.STATUS_NAMES[rc] == "SINT_ERR_CUDA"
+    # the next call's launches succeed, and it must say so
+    op.fill_quadrature_point_values(u)
+    op.evaluate_nonlinear_residual(z, u, 1)
