@@ -633,15 +633,21 @@ namespace sint
   }
 
   // The FP64 matrix in the interface's order: A[(k * 4 + e) * ld + n],
-  // neighbour k = (dx + 1) + 3 (dy + 1) (+ 9 (dz + 1)).
+  // neighbour k = (dx + 1) + 3 (dy + 1) (+ 9 (dz + 1)); zeros behind the last node.
   template <int DIM>
   __global__ void __launch_bounds__(256) ch_export_kernel(const Grid g, const ColourLattice cl,
                                                           const double *__restrict__ A, double *__restrict__ out)
   {
     using S           = ChStencil<DIM>;
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= g.N)
+    if (n >= g.ld)
       return;
+    if (n >= g.N)
+      {
+        for (int i = 0; i < S::NK * 4; ++i)
+          out[i * g.ld + n] = 0.0;
+        return;
+      }
     const int x = int(n % g.nn[0]), y = int((n / g.nn[0]) % g.nn[1]);
     const int z = DIM == 3 ? int(n / ((long long)g.nn[0] * g.nn[1])) : 0;
     const int       col = (x & 1) | ((y & 1) << 1) | ((z & 1) << 2);
@@ -969,7 +975,7 @@ namespace sint
   cudaError_t ch_matrix_export(const Ctx *c, double *A, cudaStream_t s)
   {
     const Grid    &g  = c->grid;
-    const unsigned nb = (unsigned)((g.N + 255) / 256);
+    const unsigned nb = (unsigned)((g.ld + 255) / 256);
     if (g.dim == 3)
       ch_export_kernel<3><<<nb, 256, 0, s>>>(g, colour_lattice<3>(g), c->ch_A64, A);
     else
