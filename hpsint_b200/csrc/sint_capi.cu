@@ -1,5 +1,6 @@
 // C ABI of the sintering operator: context life cycle, operator and
 // preconditioner entry points.  See include/hpsint_b200.h for the contract.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -80,10 +81,28 @@ namespace sint
     return !c->cut && !c->adv && runs_fused2d(c->grid.dim, c->G, c->params.tensorial != 0, real_size);
   }
 
+  // The one-kernel loop's blocks read nodes whose results others store, so an
+  // output that is one of the inputs is formed in the tile-face partials, which
+  // this loop does not use (sint_create gives them room for a block vector),
+  // and copied from there.  The tiled kernels read a tile's own nodes and the
+  // shared ones that only the combine step writes: they run in place.
+  template <typename R>
+  static cudaError_t copy_vector(const Ctx *c, R *dst, const R *src, cudaStream_t s)
+  {
+    return cudaMemcpy2DAsync(dst, c->ld * sizeof(R), src, c->ld * sizeof(R), c->N * sizeof(R), c->C,
+                             cudaMemcpyDeviceToDevice, s);
+  }
+
   template <typename R>
   cudaError_t dispatch_jvp(const Ctx *c, const R *lin, const R *src, R *dst, cudaStream_t s)
   {
     R *part = reinterpret_cast<R *>(c->partial);
+    const bool fused = runs_fused(c, sizeof(R));
+    if (fused && (dst == src || dst == lin))
+      {
+        const cudaError_t e = dispatch_jvp<R>(c, lin, src, part, s);
+        return e == cudaSuccess ? copy_vector(c, dst, part, s) : e;
+      }
     const bool      t   = c->params.tensorial != 0;
     const CutTiles *cut = active_cut(c);
     const AdvData  *adv = active_adv(c);
@@ -96,7 +115,7 @@ namespace sint
             : launch_jvp<2, false, R>(c->G, c->grid, c->phys, lin, src, dst, part, cut, adv, s);
     if (e != cudaSuccess)
       return e;
-    if (!runs_fused(c, sizeof(R)))
+    if (!fused)
       e = c->grid.dim == 3 ? launch_combine<3, R>(c->C, c->grid, part, dst, active_tile_union(c), s, nullptr)
                            : launch_combine<2, R>(c->C, c->grid, part, dst, active_tile_union(c), s, nullptr);
     if (e != cudaSuccess)
@@ -117,6 +136,15 @@ namespace sint
     const bool      t   = c->params.tensorial != 0;
     const CutTiles *cut = active_cut(c);
     const AdvData  *adv = active_adv(c);
+    const bool      fused = runs_fused(c, sizeof(double));
+    bool            in_place = dst == src;
+    for (int i = 0; wtd == 2 && i < c->phys.order; ++i)
+      in_place = in_place || dst == hist[i];
+    if (fused && in_place)
+      {
+        const cudaError_t e = dispatch_residual(c, wtd, src, hist, c->partial, s, hooks);
+        return e == cudaSuccess ? copy_vector(c, dst, c->partial, s) : e;
+      }
     Phys            ph  = c->phys;
     const bool      epi_after = hooks && hooks->epilogue && c->grid.periodic;
     if (hooks)
@@ -134,7 +162,7 @@ namespace sint
             : launch_residual<2, false>(c->G, wtd, c->grid, ph, src, hist, dst, c->partial, cut, adv, s);
     if (e != cudaSuccess)
       return e;
-    if (!runs_fused(c, sizeof(double)))
+    if (!fused)
       e = c->grid.dim == 3 ?
             launch_combine<3, double>(c->C, c->grid, c->partial, dst, active_tile_union(c), s, &ph.hooks) :
             launch_combine<2, double>(c->C, c->grid, c->partial, dst, active_tile_union(c), s, &ph.hooks);
@@ -391,9 +419,9 @@ int sint_create(const sint_mesh *mesh, const sint_params *params, sint_ctx **out
   const Grid &g  = c->grid;
   const long long nt = g.n_tiles;
   const int box   = mesh->dim == 3 ? Tile<3>::BOX : Tile<2>::BOX;
-  c->partial_bytes = size_t(nt) * size_t(c->G + 4) * size_t(box) * sizeof(double);
-  cudaError_t e;
   const size_t vec64 = size_t(c->C) * g.ld * sizeof(double);
+  c->partial_bytes   = std::max(size_t(nt) * size_t(c->G + 4) * size_t(box) * sizeof(double), vec64);
+  cudaError_t e;
   const size_t pcsz  = size_t(c->G + 4) * g.ld;
   if ((e = cudaMalloc(&c->lin64, vec64)) != cudaSuccess || (e = cudaMalloc(&c->lin32, vec64 / 2)) != cudaSuccess ||
       (e = cudaMalloc(&c->partial, c->partial_bytes)) != cudaSuccess ||
