@@ -481,7 +481,8 @@ int sint_destroy(sint_ctx *c)
   cudaFree(c->adv_slots);
   cudaFree(c->ch_A64);
   cudaFree(c->ch_A32);
-  cudaFree(c->ch_scratch);
+  if (c->ch_scratch != c->partial)
+    cudaFree(c->ch_scratch);
   cudaFree(c->pc_raw);
   cudaFree(c->pc_inv64);
   cudaFree(c->pc_inv32);

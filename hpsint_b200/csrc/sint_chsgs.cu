@@ -839,26 +839,69 @@ namespace sint
     return cudaErrorInvalidValue;
   }
 
-  // Cell layers per slab: as many as fit in this much scratch, at least one.
-  // Small slabs that stay in L2 lose more to short launches than they save in
-  // HBM traffic: set-up of 118^3 cells, 6 grains, with 64 / 256 / 576 / 1024
-  // MiB 5.13 / 3.56 / 3.35 / 3.41 ms (eight colour launches that updated the
-  // matrix in place, and the separate diagonal kernel: 9.4 ms).
-    constexpr size_t CH_SCRATCH_BYTES = size_t(512) << 20;
+  // Scratch of the assembly: as many cell layers per slab as fit in this many
+  // bytes (of a context's own, kept for its later set-ups), at least one, which
+  // takes two node layers.  Small slabs that stay in L2 lose more to short
+  // launches than they save in HBM traffic: set-up of 118^3 cells, 6 grains,
+  // with 64 / 256 / 576 / 1024 MiB 5.13 / 3.56 / 3.35 / 3.41 ms (eight colour
+  // launches that updated the matrix in place, and the separate diagonal
+  // kernel: 9.4 ms).
+  constexpr size_t CH_SCRATCH_BYTES = size_t(512) << 20;
 
   template <int DIM>
-  static ChScratch scratch_layout(const Grid &g, int G)
+  static long long scratch_planes(int G)
   {
-    constexpr int   NQ = 1 << DIM;
-    ChScratch       sc{};
-    sc.pitch                = (g.nn[0] + 1) / 2 * 2;
-    sc.layer                = DIM == 3 ? (long long)sc.pitch * g.nn[1] : sc.pitch;
-    const long long planes  = 3 * NQ * NQ + NQ * G;
-    const long long slabs   = (long long)(CH_SCRATCH_BYTES / (size_t(planes * sc.layer) * sizeof(double)));
-    const int       layers  = g.n[DIM - 1];
-    sc.ring                 = int(slabs < 2 ? 2 : (slabs < layers + 1 ? slabs : layers + 1));
-    sc.plane                = sc.layer * sc.ring;
+    constexpr int NQ = 1 << DIM;
+    return 3 * NQ * NQ + NQ * G;
+  }
+
+  // Layout in `bytes` of scratch; the ring holds at least two layers, even if
+  // they take more (scratch_bytes).
+  template <int DIM>
+  static ChScratch scratch_layout(const Grid &g, int G, size_t bytes)
+  {
+    ChScratch sc{};
+    sc.pitch              = (g.nn[0] + 1) / 2 * 2;
+    sc.layer              = DIM == 3 ? (long long)sc.pitch * g.nn[1] : sc.pitch;
+    const long long slabs = (long long)(bytes / (size_t(scratch_planes<DIM>(G) * sc.layer) * sizeof(double)));
+    const int       layers = g.n[DIM - 1];
+    sc.ring               = int(slabs < 2 ? 2 : (slabs < layers + 1 ? slabs : layers + 1));
+    sc.plane              = sc.layer * sc.ring;
     return sc;
+  }
+  template <int DIM>
+  static size_t scratch_bytes(const Grid &g, int G, size_t bytes)
+  {
+    return size_t(scratch_layout<DIM>(g, G, bytes).plane) * size_t(scratch_planes<DIM>(G)) * sizeof(double);
+  }
+
+  // The scratch of a context, at its first set-up.  Where the device has no
+  // room for it, the set-up works in smaller slabs: in the tile-face partials,
+  // which no other call of the context uses meanwhile, if they hold two layers
+  // (3D: from 16 cell layers on for 12 grains, from 35 for one; 2D: from 10 and
+  // 17 rows), else in an allocation of two layers.
+  template <int DIM>
+  static cudaError_t scratch_alloc(Ctx *c)
+  {
+    const size_t want = scratch_bytes<DIM>(c->grid, c->G, CH_SCRATCH_BYTES);
+    const size_t two  = scratch_bytes<DIM>(c->grid, c->G, 0);
+    cudaError_t  e    = cudaMalloc(&c->ch_scratch, want);
+    c->ch_scratch_bytes = want;
+    if (e == cudaErrorMemoryAllocation && two <= c->partial_bytes)
+      {
+        c->ch_scratch       = c->partial;
+        c->ch_scratch_bytes = c->partial_bytes;
+        e                   = cudaSuccess;
+      }
+    else if (e == cudaErrorMemoryAllocation && two < want)
+      {
+        e                   = cudaMalloc(&c->ch_scratch, two);
+        c->ch_scratch_bytes = two;
+      }
+    cudaGetLastError(); // a refused allocation is not the next launch's error
+    if (e != cudaSuccess)
+      c->ch_scratch = nullptr;
+    return e;
   }
 
   template <int DIM, bool TENS, bool CUT, bool ADV>
@@ -866,7 +909,7 @@ namespace sint
   {
     const Grid         &g  = c->grid;
     const ColourLattice cl = colour_lattice<DIM>(g);
-    ChScratch           sc = scratch_layout<DIM>(g, c->G);
+    ChScratch           sc = scratch_layout<DIM>(g, c->G, c->ch_scratch_bytes);
     sc.s                   = c->ch_scratch;
     const ChOut o{c->ch_A64, c->ch_A32, c->pc_raw, c->pc_inv64, c->pc_inv32};
     const int   n = g.n[DIM - 1];
@@ -912,20 +955,14 @@ namespace sint
       }
     const bool          d3 = c->grid.dim == 3;
     const ColourLattice cl = d3 ? colour_lattice<3>(c->grid) : colour_lattice<2>(c->grid);
-    const ChScratch     sc = d3 ? scratch_layout<3>(c->grid, c->G) : scratch_layout<2>(c->grid, c->G);
-    const int           nq = d3 ? 8 : 4;
     const size_t        n64 = size_t(cl.groups) * 128 * (d3 ? ChStencil<3>::slots(true) : ChStencil<2>::slots(true));
     const size_t        n32 = size_t(cl.groups) * 128 * (d3 ? ChStencil<3>::slots(false) : ChStencil<2>::slots(false));
-    const size_t        nsc = size_t(sc.plane) * size_t(3 * nq * nq + nq * c->G);
     cudaError_t         e   = cudaSuccess;
-    if (!c->ch_scratch)
-      {
-        // the rows that fill up a colour's last group of 32 are never used
-        if ((!c->ch_A64 && (e = cudaMalloc(&c->ch_A64, n64 * sizeof(double))) != cudaSuccess) ||
-            (!c->ch_A32 && (e = cudaMalloc(&c->ch_A32, n32 * sizeof(float))) != cudaSuccess) ||
-            (e = cudaMalloc(&c->ch_scratch, nsc * sizeof(double))) != cudaSuccess)
-          return cuda_fail(e, "sint_precond_setup: Cahn-Hilliard matrix allocation");
-      }
+    // the rows that fill up a colour's last group of 32 are never used
+    if ((!c->ch_A64 && (e = cudaMalloc(&c->ch_A64, n64 * sizeof(double))) != cudaSuccess) ||
+        (!c->ch_A32 && (e = cudaMalloc(&c->ch_A32, n32 * sizeof(float))) != cudaSuccess) ||
+        (!c->ch_scratch && (e = d3 ? scratch_alloc<3>(c) : scratch_alloc<2>(c)) != cudaSuccess))
+      return cuda_fail(e, "sint_precond_setup: Cahn-Hilliard matrix allocation");
     e = c->grid.dim == 3 ? assemble_mob<3>(c, s) : assemble_mob<2>(c, s);
     return e == cudaSuccess ? SINT_OK : cuda_fail(e, "sint_precond_setup: Cahn-Hilliard matrix");
   }

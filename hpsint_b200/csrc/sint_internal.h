@@ -96,7 +96,8 @@ namespace sint
     bool    has_ch    = false;   // the assembled block belongs to the current set-up
     double *ch_A64     = nullptr; // 2x2 blocks of the node rows, layout and slots in sint_chsgs.cu
     float  *ch_A32     = nullptr;
-    double *ch_scratch = nullptr; // element-matrix rows of a slab of cell layers (assembly)
+    double *ch_scratch = nullptr; // element-matrix rows of a slab of cell layers (assembly); `partial` if shared
+    size_t  ch_scratch_bytes = 0;
 
     double *pc_raw   = nullptr; // (G+4) blocks: CH 2x2 entries, AC diagonal
     double *pc_inv64 = nullptr; // (G+4) blocks: CH 2x2 inverse, AC inverse diagonal

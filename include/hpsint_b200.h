@@ -208,7 +208,13 @@ int sint_precond_setup(sint_ctx *ctx, sint_stream_t stream);
  *      (sint_newton_params.right_preconditioning): with left preconditioning
  *      GMRES stops on a residual dominated by the Cahn-Hilliard rows.
  * Takes effect at the next sint_precond_setup; type 1 allocates the matrix
- * (3^dim x 4 FP64 + FP32 values per node) at its first set-up. */
+ * (4 (3^dim + 1) FP64 and 4 x 3^dim FP32 values per node, inverted centre
+ * blocks included) at its first set-up, and scratch for the assembly: the
+ * element rows of all cell layers or, where those take more, as many layers as
+ * fit in 512 MiB, at least two node layers (8 (192 + 8 G) bytes per node in 3D,
+ * 8 (48 + 4 G) in 2D).  Where the device has no room for that, the assembly
+ * uses the context's other scratch or two node layers.  Both are kept until
+ * sint_destroy. */
 int sint_set_preconditioner_type(sint_ctx *ctx, int type);
 
 /* The assembled Cahn-Hilliard block of preconditioner type 1: 3^dim x 4
