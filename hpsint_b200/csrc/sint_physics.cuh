@@ -33,17 +33,20 @@ namespace sint
     return s;
   }
 
-  // Reciprocal and inverse square root of a positive number: a hardware seed
-  // and one step of a power series in its error e,
-  //   reciprocal:          e = 1 - x y,    y <- y (1 + e + e^2 (FP64))
-  //   inverse square root: e = 1 - x y^2,  y <- y (1 + e / 2 + 3 e^2 / 8 (FP64))
-  // FP32: rcp.approx / rsqrt.approx (error ~2^-23) and the linear step, float
-  // rounding level.  FP64: rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64, which
-  // take and give doubles of full exponent range with ~20 good bits, and the
-  // quadratic step: error below 2^-52 + e^3.  Against the float seeds with a
-  // linear step and their scaling by 2^56, which these replace, that saves
-  // two conversions and one operation per reciprocal and is more exact (3e-14
-  // before).
+  // Reciprocal and inverse square root of a positive number from the hardware's
+  // approximation y, by the binomial series in its error e:
+  //   1 / x     = y (1 - e)^-1,    e = 1 - x y    ->  y (1 + e + e^2 (FP64))
+  //   x^(-1/2)  = y (1 - e)^-1/2,  e = 1 - x y^2  ->  y (1 + e / 2 + 3 e^2 / 8 (FP64))
+  // The linear step is Newton's, the quadratic one the hyperpower iteration of
+  // order three (M. Altman, Pacific J. Math. 10, 1960) and its counterpart for
+  // the root.  FP32: rcp.approx / rsqrt.approx (error ~2^-23) and the linear
+  // step, float rounding level.  FP64: rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64,
+  // which take and give doubles, and the quadratic step: relative error below
+  // 2^-52 while argument and reciprocal are normal numbers
+  // (test_gpu_point_reciprocals.py compares them with CUDA's division and rsqrt).
+  // Against the float seeds with a linear step and their scaling by 2^56, which
+  // these replace, that saves two conversions and one operation per reciprocal
+  // and is more exact (3e-14 before).
   __device__ __forceinline__ float rcp_seed(float x)
   {
     float y;
