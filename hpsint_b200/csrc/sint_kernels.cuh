@@ -1221,18 +1221,21 @@ namespace sint
     const long long          i1 = CUT ? (long long)ct.range[G + 1] : g.n_tiles;
     // The next tile's nodal values (this thread's box node, every NG-th
     // component) wait in registers while this tile's sums are stored: the
-    // history is combined with arithmetic, so cp.async cannot stage it.
-    constexpr int NV = (C + T::NG - 1) / T::NG;
-    R             rv[NV], rh[WTD == 2 ? NV : 1][3];
-    auto          load = [&](long long idx) {
-      if (idx >= i1 || !np.active)
+    // history is combined with arithmetic, so cp.async cannot stage it.  Not
+    // with at most one grain, where finding the next tile ahead costs more than
+    // the few loads it hides (one grain, scalar, no history, 96^3 cells: 178 us
+    // ahead, 168 at the tile; cut-off class without grains, with advection, 136
+    // and 125 us).
+    constexpr bool AHEAD = G > 1;
+    constexpr int  NV    = (C + T::NG - 1) / T::NG;
+    R              rv[NV], rh[WTD == 2 ? NV : 1][3];
+    auto           load = [&](const TileCoord &tc, bool interior, long long node0, unsigned long long gl) {
+      if (!np.active)
         return;
-      const unsigned long long gl   = CUT ? ct.tile_grains[idx] : 0ull;
-      const TileCoord          tc   = tile_coord_of<DIM>(g, CUT ? (long long)ct.tiles[idx] : idx);
       // in an interior tile the box node exists and reads itself
       bool      inside = true;
-      long long lidx   = tile_node0(g, tc) + np.off;
-      if (!tile_interior<DIM>(g, tc))
+      long long lidx   = node0 + np.off;
+      if (!interior)
         {
           const BoxNode<DIM> bn(g, tc);
           inside = bn.inside;
@@ -1257,7 +1260,14 @@ namespace sint
             }
         }
     };
-    load(i0 + blockIdx.x);
+    auto load_ahead = [&](long long idx) {
+      if (idx >= i1)
+        return;
+      const TileCoord tc = tile_coord_of<DIM>(g, CUT ? (long long)ct.tiles[idx] : idx);
+      load(tc, tile_interior<DIM>(g, tc), tile_node0(g, tc), CUT ? ct.tile_grains[idx] : 0ull);
+    };
+    if constexpr (AHEAD)
+      load_ahead(i0 + blockIdx.x);
     for (long long idx = i0 + blockIdx.x; idx < i1; idx += gridDim.x)
       {
         const long long          tile = CUT ? (long long)ct.tiles[idx] : idx;
@@ -1267,6 +1277,8 @@ namespace sint
         const bool               interior = tile_interior<DIM>(g, tc);
         const long long          node0    = tile_node0(g, tc);
         const unsigned m = CUT ? local_mask<G>(cell_mask<DIM>(ct.cell_mask, g, tc, threadIdx.x % T::CELLS), gl) : ~0u;
+        if constexpr (!AHEAD)
+          load(tc, interior, node0, gl);
         if (np.active)
 #pragma unroll
           for (int n = 0; n < NV; ++n)
@@ -1303,7 +1315,8 @@ namespace sint
         __syncthreads();
         phase_integrate<DIM, G, FM, R, CUT, ADV>(p, g, k, tc, P, s_u, K, m, A_vel, A_has);
         __syncthreads();
-        load(idx + gridDim.x);
+        if constexpr (AHEAD)
+          load_ahead(idx + gridDim.x);
         if (interior)
           sum_and_store_interior<DIM>(K, C, g, tc.linear, np, node0, dst, partial, gl, CUT, ct.c_all, tm, &ph.hooks);
         else
