@@ -306,6 +306,15 @@ namespace sint
     return launch_residual_w<DIM, TENS, CUT, 2, ADV>(G, g, p, src, hist, dst, partial, ct, adv, s, sibling);
   }
 
+  // With advection in 3D the class without grains is a block kernel that is
+  // most of the call.  On large meshes it runs faster by itself than beside the
+  // other classes' last blocks, whose shared-memory carveout it inherits (an SM
+  // changes it only while idle): 128^3 cells, 2 grains, scalar, with history 474
+  // us, beside them 540 to 584; tensorial without history 459 and 505.  On small
+  // ones it hides their tails (64 x 56 x 48 cells, 9 grains 116 us, one class
+  // after the other 152).
+  constexpr long long CLASS0_BESIDE_TILES = 12288;
+
   template <int DIM, bool TENS, bool ADV>
   cudaError_t launch_residual_impl(int G, int wtd, const Grid &g, const Phys &p, const double *src,
                                    const double *const *hist, double *dst, double *partial, const CutTiles *cut,
@@ -314,9 +323,12 @@ namespace sint
     if (cut)
       {
         for (int K = G; K >= 0; --K) // as the Jacobian product
-          if (const cudaError_t e =
-                launch_residual_c<DIM, TENS, true, ADV>(K, wtd, g, p, src, hist, dst, partial, *cut, adv, s, K < G))
-            return e;
+          {
+            const bool beside = K < G && !(ADV && DIM == 3 && K == 0 && g.n_tiles > CLASS0_BESIDE_TILES);
+            if (const cudaError_t e =
+                  launch_residual_c<DIM, TENS, true, ADV>(K, wtd, g, p, src, hist, dst, partial, *cut, adv, s, beside))
+              return e;
+          }
         return cudaSuccess;
       }
     return launch_residual_c<DIM, TENS, false, ADV>(G, wtd, g, p, src, hist, dst, partial, CutTiles(), adv, s);
