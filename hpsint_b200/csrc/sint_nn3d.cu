@@ -243,44 +243,73 @@ namespace sint
       const long long zs = (long long)a.cout * hw;
       float          *op = a.out + ((long long)s * D2 + z0) * zs + pix;
       const float    *ap = a.addend ? a.addend + ((long long)(s / a.addend_group) * D2 + z0) * zs + pix : nullptr;
-      constexpr int CE = COUT < 8 ? COUT : 8;
-      // the addends of CE channels are loaded together, and read-only so that they
-      // may go ahead of the stores before them: one at a time each load
-      // waited for its turn behind a store
-#pragma unroll
-      for (int z = 0; z < ZB; ++z)
+      auto            value = [&](int z, int co) -> float {
+        if constexpr (PAIRS)
+          return co & 1 ? acc2[z][co / 2].y : acc2[z][co / 2].x;
+        else
+          return acc[z][co];
+      };
+      if (!ap && !a.accumulate)
         {
-          if (z0 + z > a.D)
-            break;
 #pragma unroll
-          for (int c0 = 0; c0 < COUT; c0 += CE)
+          for (int z = 0; z < ZB; ++z)
             {
-              float add[CE];
+              if (z0 + z > a.D)
+                break;
 #pragma unroll
-              for (int c = 0; c < CE; ++c)
+              for (int co = 0; co < COUT; ++co)
                 {
-                  const int co = c0 + c;
-                  add[c]       = ap && co < a.cout ? __ldg(ap + z * zs + co * hw) : 0.f;
-                  if (a.accumulate && co < a.cout)
-                    add[c] += op[z * zs + co * hw];
-                }
-#pragma unroll
-              for (int c = 0; c < CE; ++c)
-                {
-                  const int co = c0 + c;
                   if (co >= a.cout)
                     break;
-                  float v;
-                  if constexpr (PAIRS)
-                    v = co & 1 ? acc2[z][co / 2].y : acc2[z][co / 2].x;
-                  else
-                    v = acc[z][co];
+                  float v = value(z, co);
                   if (a.bias)
-                    v += __ldg(a.bias + co);
-                  v += add[c];
+                    v += COUT == 8 ? __ldg(a.bias + co) : a.bias[co];
                   if (a.leaky && v < 0.f)
                     v *= a.slope;
                   op[z * zs + co * hw] = v;
+                }
+            }
+        }
+      else
+        {
+          // the addends of CE channels are loaded together, and read-only so that
+          // they may go ahead of the stores before them: one at a time each load
+          // waited for its turn behind a store.  (Without addends this form costs
+          // up to 3 us a launch: 2 windows of 24 x 64 x 64, 2 to 8 channels 14.2
+          // us, 11.6 as above, where the bias through the read-only path gained 3
+          // % at 8 output channels and lost up to 5 % at others.)
+          constexpr int CE = COUT < 8 ? COUT : 8;
+#pragma unroll
+          for (int z = 0; z < ZB; ++z)
+            {
+              if (z0 + z > a.D)
+                break;
+#pragma unroll
+              for (int c0 = 0; c0 < COUT; c0 += CE)
+                {
+                  float add[CE];
+#pragma unroll
+                  for (int c = 0; c < CE; ++c)
+                    {
+                      const int co = c0 + c;
+                      add[c]       = ap && co < a.cout ? __ldg(ap + z * zs + co * hw) : 0.f;
+                      if (a.accumulate && co < a.cout)
+                        add[c] += op[z * zs + co * hw];
+                    }
+#pragma unroll
+                  for (int c = 0; c < CE; ++c)
+                    {
+                      const int co = c0 + c;
+                      if (co >= a.cout)
+                        break;
+                      float v = value(z, co);
+                      if (a.bias)
+                        v += __ldg(a.bias + co);
+                      v += add[c];
+                      if (a.leaky && v < 0.f)
+                        v *= a.slope;
+                      op[z * zs + co * hw] = v;
+                    }
                 }
             }
         }
