@@ -6,7 +6,8 @@
 // memory budget is fixed up front.  sint_jvp_f64_noalloc serves them: it
 // takes the mesh, the parameters, the time weights and the linearisation
 // point directly (no context), and the only scratch the product needs -- the
-// tile-face partial sums between the cell kernel and the combine kernel --
+// tile-face partial sums between the cell kernel and the combine kernel, or in
+// the one-kernel 2D product the result of a call whose dst is lin or src --
 // lives in a fixed device array of this file instead of an allocation.
 #include <mutex>
 #include <string>
@@ -16,8 +17,8 @@
 
 namespace sint
 {
-  // Scratch of the allocation-free product: tile-face partial sums, at most
-  // SINT_NOALLOC_SCRATCH_BYTES.  Every GPU that loads this library holds it
+  // Scratch of the allocation-free product: tile-face partial sums or a block
+  // vector, at most SINT_NOALLOC_SCRATCH_BYTES.  Every GPU that loads this library holds it
   // until the process exits.  All calls share it.
   static __device__ __align__(256) double noalloc_scratch[SINT_NOALLOC_SCRATCH_BYTES / sizeof(double)];
 
@@ -75,6 +76,8 @@ extern "C" int sint_jvp_f64_noalloc(const sint_mesh *mesh, const sint_params *pa
   Ctx c;
   if (int rc = describe_operator(mesh, params, &c))
     return rc;
+  // one limit for every call of a mesh: the partials, which are no smaller than a
+  // block vector on any mesh that comes near it
   const int       box   = mesh->dim == 3 ? Tile<3>::BOX : Tile<2>::BOX;
   const long long need  = c.grid.n_tiles * (long long)c.C * box * (long long)sizeof(double);
   if (need > (long long)SINT_NOALLOC_SCRATCH_BYTES)

@@ -113,7 +113,8 @@ int sint_set_linearization_point(sint_ctx *ctx, const double *u, sint_stream_t s
  * 0 drops the time terms, 1 keeps w0*u only, 2 adds the BDF history
  * sum_i w_hist[i] * hist[i].  hist is a HOST array of `order` device pointers
  * to old solutions (SolutionHistory::get_old_solutions); ignored unless
- * with_time_derivative == 2.  dst is overwritten. */
+ * with_time_derivative == 2.  dst is overwritten; it may be src or one of
+ * hist. */
 int sint_residual_f64(sint_ctx *ctx, double *dst, const double *src, const double *const *hist,
                       int with_time_derivative, sint_stream_t stream);
 
@@ -147,7 +148,8 @@ int sint_residual_f64_hooks(sint_ctx *ctx, double *dst, const double *src, const
 
 /* OperatorBase::vmult -> SinteringOperatorGeneric::vmult_internal
  * (operator_base.h:294-353, operator_sintering_generic.h:539-606):
- * dst = J(u_lin) src in FP64.  dst is overwritten. */
+ * dst = J(u_lin) src in FP64.  dst is overwritten; it may be src,
+ * but for periodic meshes. */
 int sint_jvp_f64(sint_ctx *ctx, double *dst, const double *src, sint_stream_t stream);
 
 /* Same product in FP32 with FP32 accumulation, linearised at the FP32 shadow. */
@@ -161,10 +163,12 @@ int sint_jvp_f32(sint_ctx *ctx, float *dst, const float *src, sint_stream_t stre
  * (w0, w_alg as in sint_set_time_weights), the linearisation point `lin` and
  * the direction `src` (C blocks each, the layout sint_dof_layout reports) and
  * owns `dst`; the result equals sint_jvp_f64 on a context with the same state.
- * The product's only scratch, the partial sums on tile faces, lives in a
- * fixed device array of SINT_NOALLOC_SCRATCH_BYTES that every GPU loading the
- * library holds until exit; meshes needing more return SINT_ERR_ARG.  The
- * need is 600 * (G + 2) bytes per 4 x 4 x 2 cells in 3D and 648 * (G + 2)
+ * The product's only scratch, the partial sums on tile faces (in 2D mostly
+ * unused: there one kernel finishes every node, and needs the scratch when dst
+ * is lin or src), lives in a fixed device array of SINT_NOALLOC_SCRATCH_BYTES
+ * that every GPU loading the library holds until exit; meshes whose partial
+ * sums would need more return SINT_ERR_ARG, whatever the call uses.  That need
+ * is 600 * (G + 2) bytes per 4 x 4 x 2 cells in 3D and 648 * (G + 2)
  * bytes per 8 x 8 cells in 2D: with G = 4, up to 64 x 64 x 36 cells in 3D or
  * 520 x 520 cells in 2D.  The first call on a device looks up the array's device address
  * (cudaGetSymbolAddress) with that device current, so make it before any
@@ -191,7 +195,8 @@ int sint_jvp_f64_noalloc(const sint_mesh *mesh, const sint_params *params, doubl
  * blocks include the advection terms of the current velocity table
  * (precondition_advection_ch / _ac, operator_sintering_generic.h:800-850); on a
  * periodic mesh the slave rows are condensed into their masters and get the
- * identity. */
+ * identity.  A set-up that fails leaves no preconditioner: the applies return
+ * SINT_ERR_NOT_READY until one succeeds. */
 int sint_precond_setup(sint_ctx *ctx, sint_stream_t stream);
 
 /* Block 0 of the preconditioner (BlockPreconditioner2Data::block_0,
