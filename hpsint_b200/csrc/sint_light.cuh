@@ -228,6 +228,10 @@ namespace sint
             for (int qy = 0; qy < 2; ++qy)
               {
                 const R py1 = qy ? k.x1 : k.x0, py0 = qy ? k.x0 : k.x1;
+                // sums of this line of two points, to its ends in x: values, x flux,
+                // y flux, z flux, mu row
+                R lv[2], lx = R(0), ly[2], lz[2], lm[2];
+                lv[0] = lv[1] = ly[0] = ly[1] = lz[0] = lz[1] = lm[0] = lm[1] = R(0);
 #pragma unroll
                 for (int qx = 0; qx < 2; ++qx)
                   {
@@ -244,32 +248,13 @@ namespace sint
                       o[2] = xy(dz[f]) * k.ih[2];
                     };
                     auto emit = [&](int res, R v) {
-                      if (res == 0)
-                        {
-#pragma unroll
-                          for (int c = 0; c < 4; ++c)
-                            cv[c] += (((c & 1) ? px1 : px0) * ((c >> 1) ? py1 : py0)) * v;
-                        }
-                      else if (res == 1)
-                        {
-                          cv[0] -= (k.ih[0] * py0) * v;
-                          cv[1] += (k.ih[0] * py0) * v;
-                          cv[2] -= (k.ih[0] * py1) * v;
-                          cv[3] += (k.ih[0] * py1) * v;
-                        }
-                      else if (res == 2)
-                        {
-                          cv[0] -= (k.ih[1] * px0) * v;
-                          cv[2] += (k.ih[1] * px0) * v;
-                          cv[1] -= (k.ih[1] * px1) * v;
-                          cv[3] += (k.ih[1] * px1) * v;
-                        }
+                      if (res == 1)
+                        lx += v;
                       else
                         {
-                          R(&o)[4] = res == 3 ? cz : mv;
-#pragma unroll
-                          for (int c = 0; c < 4; ++c)
-                            o[c] += (((c & 1) ? px1 : px0) * ((c >> 1) ? py1 : py0)) * v;
+                          R(&o)[2] = res == 0 ? lv : (res == 2 ? ly : (res == 3 ? lz : lm));
+                          o[0] += px0 * v;
+                          o[1] += px1 * v;
                         }
                     };
                     const R c = xy(a[0]);
@@ -298,6 +283,16 @@ namespace sint
                           return v;
                         },
                         emit);
+                  }
+                lv[0] -= k.ih[0] * lx;
+                lv[1] += k.ih[0] * lx;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                  {
+                    const R py = (c >> 1) ? py1 : py0;
+                    cv[c] += py * lv[c & 1] + ((c >> 1) ? k.ih[1] : -k.ih[1]) * ly[c & 1];
+                    cz[c] += py * lz[c & 1];
+                    mv[c] += py * lm[c & 1];
                   }
               }
             const R w0 = pz0 * k.JxW, w1 = pz1 * k.JxW, wz = k.ih[2] * k.JxW;
