@@ -676,9 +676,11 @@ namespace sint
   // (2, 6, 18 neighbours) are loaded before the wait; all of them take 128
   // registers, which pays while the colour is one wave of blocks (FP32 apply
   // at 48^3 cells 36.5 us, PRE = 2 48.7 us, PRE = 0 95.1 us; at 96^3 111.8 /
-  // 94.8 / 124.4 us; at 192^3 756 / 655 / 690 us; entry-major rows without
-  // programmatic launches took 930 us there).  The first launch of an apply (ac_blocks > 0) also does the grain
-  // rows z = inverse diagonal * r in its blocks behind the colour's.
+  // 94.8 / 124.4 us; at 192^3 756 / 655 / 690 us).  With the rule as it stands
+  // the apply takes 632 / 661 / 705 us at 192^3 cells with 4 / 6 / 9 grains;
+  // entry-major rows without programmatic launches took 951 us with 9.  The
+  // first launch of an apply (ac_blocks > 0) also does the grain rows z =
+  // inverse diagonal * r in its blocks behind the colour's.
   constexpr int       SGS_THREADS  = 128;
   constexpr long long SGS_WAVE_F32 = 148 * 4 * SGS_THREADS, SGS_WAVE_F64 = 148 * 2 * SGS_THREADS;
 
@@ -848,9 +850,9 @@ namespace sint
   // bytes (of a context's own, kept for its later set-ups), at least one, which
   // takes two node layers.  Small slabs that stay in L2 lose more to short
   // launches than they save in HBM traffic: set-up of 118^3 cells, 6 grains,
-  // with 64 / 256 / 576 / 1024 MiB 5.13 / 3.56 / 3.35 / 3.41 ms (eight colour
-  // launches that updated the matrix in place, and the separate diagonal
-  // kernel: 9.4 ms).
+  // with 64 / 256 / 576 / 1024 MiB 5.13 / 3.56 / 3.35 / 3.41 ms when the bound was
+  // chosen, 2.96 ms with these 512 MiB today (eight colour launches that updated
+  // the matrix in place, and the separate diagonal kernel: 9.4 ms).
   constexpr size_t CH_SCRATCH_BYTES = size_t(512) << 20;
 
   template <int DIM>

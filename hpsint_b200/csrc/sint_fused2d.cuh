@@ -13,10 +13,10 @@
 // busy at 512 x 512 cells, the rest is the ramp of each block's loads and the
 // last wave).  16 x 8 threads recompute 22 % of the cells; 16 x 16 recompute
 // 14 % but balance worse over the SMs and overlap loads and arithmetic less
-// (two blocks per SM instead of four): 512 x 512, FP32 scalar J v of 8 grains
-// 35.1 us against 39.9 us; 256 x 128, FP64 tensorial J v of 3 grains 10.6 us
-// against 12.6 us.  The tiled kernels with their combine launch took 51.5 us
-// and 16.6 us.
+// (two blocks per SM instead of four): when the tile was chosen, 512 x 512, FP32
+// scalar J v of 8 grains 35.1 us against 39.9 us; 256 x 128, FP64 tensorial J v
+// of 3 grains 10.6 us against 12.6 us.  Those two take 31.5 and 7.1 us today;
+// the tiled kernels with their combine launch took 55.3 and 11.8 us.
 #pragma once
 
 #include "sint_kernels.cuh"

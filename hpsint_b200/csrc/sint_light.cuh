@@ -78,7 +78,8 @@ namespace sint
   // product 239, the FP64 residual fits 168.  (Tried on the FP32 product of a
   // 256^3 packing, all classes together: packed FP32 pairs of tiles, 255
   // registers, 2.41 ms, 168 with spills 2.48 ms; one line of two points at a
-  // time, 96 registers, 2.36 ms; this form 2.21 ms.)
+  // time, 96 registers, 2.36 ms; this form 2.21 ms, and 2.09 ms since the classes
+  // run beside one another.)
   template <typename R, int MODE>
   constexpr int light_blocks()
   {

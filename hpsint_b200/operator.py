@@ -96,7 +96,8 @@ def bdf_weights(order, dt):
 # A product of a small mesh is shorter on the GPU than its call: pointers go to
 # the library as plain integers (its argument types are declared) and the
 # current stream is read as a handle, without a Stream object (FP64 J v of 256 x
-# 128 cells, call after call, with an ordinary launch: 9.0 -> 8.5 us, small residual 10.6 -> 6.0 us).
+# 128 cells, call after call, with an ordinary launch: 9.0 -> 8.5 us; the small
+# residual 10.6 -> 6.0 us together with its dependent launch).
 def _ptr(t):
     return t.data_ptr()
 
