@@ -253,15 +253,20 @@ namespace sint
   // With more, the early blocks are spread over the SMs by what the grid before
   // leaves free, and the fullest SM decides: 710 blocks 5.6 -> 7.4 us, 1029
   // blocks 8.2 -> 11.0.  The next launch is let go only once this grid's inputs
-  // are there; let go at its start, two of them pile up (472 blocks 6.3 us).
+  // are there; let go at its start, two of them pile up (472 blocks 6.3 us).  The
+  // ordinary launch goes without both calls (FP32, one grain, 3566 blocks 5.0 us
+  // with them, 4.5 without).
   constexpr unsigned APPLY_DEPENDENT_BLOCKS = 4 * 148;
 
-  template <typename R>
+  template <typename R, bool DEPENDENT>
   __global__ void precond_apply_kernel(long long N, long long ld, int G, const R *__restrict__ inv,
                                        const R *__restrict__ r, R *__restrict__ z)
   {
-    cudaGridDependencySynchronize();
-    cudaTriggerProgrammaticLaunchCompletion();
+    if constexpr (DEPENDENT)
+      {
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+      }
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N)
       return;
@@ -276,8 +281,9 @@ namespace sint
   static cudaError_t apply_node_blocks(const Ctx *c, const R *inv, const R *r, R *z, cudaStream_t s)
   {
     const unsigned nb = (unsigned)((c->N + 255) / 256);
-    return launch_dependent_if(nb <= APPLY_DEPENDENT_BLOCKS, precond_apply_kernel<R>, dim3(nb), 256, 0, s, c->N, c->ld,
-                               c->G, inv, r, z);
+    const bool     dep = nb <= APPLY_DEPENDENT_BLOCKS;
+    return launch_dependent_if(dep, dep ? precond_apply_kernel<R, true> : precond_apply_kernel<R, false>, dim3(nb), 256,
+                               0, s, c->N, c->ld, c->G, inv, r, z);
   }
 
   __global__ void f64_to_f32_kernel(long long n, const double *__restrict__ x, float *__restrict__ y)
